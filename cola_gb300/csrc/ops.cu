@@ -87,71 +87,6 @@ __global__ void __launch_bounds__(256) dense_gemv_kernel(const S* __restrict__ A
   }
 }
 
-// Dense, many columns: 64x64 output tile, 16-deep k-slices through shared memory,
-// 256 threads each owning a 4x4 micro-tile.  blockIdx.z = batch.
-template <class T, class S>
-__global__ void __launch_bounds__(256) dense_gemm_kernel(const S* __restrict__ A, int64_t lda, int64_t M,
-                                                         int64_t K, const T* __restrict__ X, int64_t ldx,
-                                                         int64_t bsx, T* __restrict__ Y, int64_t ldy,
-                                                         int64_t bsy, int64_t N, T alpha, T beta,
-                                                         const int* skip) {
-  if (skip && *skip) return;
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ T As[BK][BM + 1];
-  __shared__ T Xs[BK][BN];
-  const int64_t b = blockIdx.z;
-  X += b * bsx;
-  Y += b * bsy;
-  const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  T acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
-  for (int64_t k0 = 0; k0 < K; k0 += BK) {
-    // A tile: BM x BK, 1024 elements, 4 per thread
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int idx = threadIdx.x + r * 256;
-      const int mm = idx / BK, kk = idx % BK;
-      const int64_t gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? cvt<T>(A[gm * lda + gk]) : T(0);
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int idx = threadIdx.x + r * 256;
-      const int kk = idx / BN, nn = idx % BN;
-      const int64_t gk = k0 + kk, gn = n0 + nn;
-      Xs[kk][nn] = (gk < K && gn < N) ? X[gk * ldx + gn] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      T av[4], xv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) xv[j] = Xs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * xv[j];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t gn = n0 + tx * 4 + j;
-      if (gn < N) Y[gm * ldy + gn] = combine(acc[i][j], alpha, beta, Y + gm * ldy + gn);
-    }
-  }
-}
-
 // CSR, one column: TPR lanes per row, lanes stride over the row's entries.
 template <class T, class S, int TPR>
 __global__ void __launch_bounds__(256) csr_spmv_kernel(const int32_t* __restrict__ indptr,
@@ -439,9 +374,7 @@ static int launch_dense(const colagb_op_node& nd, const T* X, int64_t ldx, int64
       default: dense_gemv_kernel<T, S, 4><<<grid, 256, 0, st>>>(A, nd.ld, nd.rows, nd.cols, X, ldx, bsx, Y, ldy, bsy, alpha, beta, skip); break;
     }
   } else {
-    dim3 grid((unsigned)ceil_div(k, 64), (unsigned)ceil_div(nd.rows, 64), (unsigned)batch);
-    dense_gemm_kernel<T, S><<<grid, 256, 0, st>>>(A, nd.ld, nd.rows, nd.cols, X, ldx, bsx, Y, ldy, bsy, k, alpha,
-                                                  beta, skip);
+    return dense_contract<T, S>(A, nd.ld, nd.rows, nd.cols, X, bsx, ldx, Y, bsy, ldy, batch, k, alpha, beta, skip, st);
   }
   COLAGB_CUDA(cudaGetLastError());
   return COLAGB_OK;
@@ -548,6 +481,20 @@ static bool kron_on_tensor_cores(int32_t precision, const colagb_op_node& f, int
   return true;
 }
 
+// dense_contract of a Dense node in its storage type.
+template <class T>
+static int contract_leaf(const colagb_op_node& f, const T* X, int64_t x_p, int64_t x_k, T* Y, int64_t y_p, int64_t y_m,
+                         int64_t P, int64_t q, T alpha, T beta, const int* skip, cudaStream_t st) {
+#define COLAGB_CONTRACT(S)                                                                                        \
+  return dense_contract<T, S>(static_cast<const S*>(f.data), f.ld, f.rows, f.cols, X, x_p, x_k, Y, y_p, y_m, P, q, \
+                              alpha, beta, skip, st)
+  if (f.dtype == COLAGB_F32) COLAGB_CONTRACT(float);
+  if (f.dtype == COLAGB_BF16) COLAGB_CONTRACT(__nv_bfloat16);
+  if constexpr (std::is_same<T, double>::value) COLAGB_CONTRACT(double);
+#undef COLAGB_CONTRACT
+  return fail(COLAGB_ERR_UNSUPPORTED, "leaf storage dtype not supported for this compute dtype");
+}
+
 template <class T>
 int op_apply(const colagb_op* op, int node, const T* X, int64_t ldx, int64_t bsx, T* Y, int64_t ldy, int64_t bsy,
              int64_t k, int64_t batch, T alpha, T beta, Bump& ws, const int* skip, cudaStream_t st) {
@@ -634,8 +581,11 @@ int op_apply(const colagb_op* op, int node, const T* X, int64_t ldx, int64_t bsx
       }
       const size_t mark = ws.used;
       T* buf[2] = {ws.take<T>((size_t)maxsz * k), ws.take<T>((size_t)maxsz * k)};
-      // scratch for the axis-swapped form of a factor with few columns per block (below)
-      T* sw[2] = {ws.take<T>((size_t)maxsz * k), ws.take<T>((size_t)maxsz * k)};
+      // scratch for the axis-swapped form of a factor that is not Dense and has few columns per block (below)
+      bool any_swap = false;
+      for (int i = 0; i < m; ++i) any_swap |= op->nodes[ch[i]].kind != COLAGB_OP_DENSE;
+      T* sw[2] = {nullptr, nullptr};
+      if (any_swap) sw[0] = ws.take<T>((size_t)maxsz * k), sw[1] = ws.take<T>((size_t)maxsz * k);
       for (int64_t b = 0; b < batch && !measuring; ++b) {
         const T* in = X + b * bsx;
         int which = 0;  // next scratch buffer to write
@@ -668,6 +618,10 @@ int op_apply(const colagb_op* op, int node, const T* X, int64_t ldx, int64_t bsx
               COLAGB_TRY(tc_contract(a_in, false, 1, pre, c[i], f.data, f.dtype, f.ld, r[i], o, 0, r[i], 1, a_f, b_f,
                                      split, ws, skip, st));
             ws.release(tmark);
+          } else if (op->nodes[ch[i]].kind == COLAGB_OP_DENSE) {
+            // one product over all pre * q columns, read and written in place
+            COLAGB_TRY(contract_leaf<T>(op->nodes[ch[i]], in, c[i] * q, q, out, r[i] * q, q, pre, q,
+                                        direct ? alpha : T(1), direct ? beta : T(0), skip, st));
           } else if (q <= 8 && pre >= 16 && pre <= 65535 && c[i] <= 65535) {
             // `pre` products of M_i with (c_i x q) blocks re-read M_i `pre` times; with the first two
             // axes swapped they are one product M_i @ (c_i x pre*q), then swapped back
