@@ -27,6 +27,7 @@
 #include <string>
 #include <vector>
 
+#include "cg_dense.cuh"
 #include "common.cuh"
 #include "ops.cuh"
 
@@ -1076,8 +1077,35 @@ static int finish_fused(const CgScalars<T>& s, colagb_cg_result* res, cudaStream
 template <class T, class S, int PK>
 static int run_fused(const CgPlan& pl, const T* B, int64_t ldb, T* X, int64_t ldx, const colagb_cg_params& prm, T* hist,
                      CgScalars<T> s, T* R, T* Pv, T* AP, colagb_cg_result* res, cudaStream_t st) {
-  FusedArgs<T, S> a;
   const colagb_op_node* leaf = pl.ff.leaf;
+  if constexpr (!(std::is_same<T, double>::value && std::is_same<S, __nv_bfloat16>::value))
+  if (leaf->kind == COLAGB_OP_DENSE && pl.n <= (1 << 20)) {
+    DenseCgArgs<T, S> d;
+    d.A = static_cast<const S*>(leaf->data);
+    d.lda = leaf->ld;
+    d.n = (int)pl.n;
+    d.k = (int)pl.k;
+    d.shift = (T)pl.ff.shift;
+    d.dinv = PK == 1 ? static_cast<const T*>(pl.pdiag->data) : nullptr;
+    d.B = B;
+    d.ldb = ldb;
+    d.X = X;
+    d.ldx = ldx;
+    d.AP = R;  // R, Pv and AP are consecutive: 3 n k >= 2 k (n + 3) entries
+    d.tol = prm.tol;
+    d.max_iters = prm.max_iters;
+    d.aligned = pl.n % 4 == 0 && leaf->ld % 4 == 0 && (uintptr_t)leaf->data % (4 * sizeof(S) < 16 ? 4 * sizeof(S) : 16) == 0;
+    d.hist = hist;
+    d.iters = s.iters;
+    d.count = s.counters + 4;
+    d.err = reinterpret_cast<int*>(s.counters + 6);
+    d.spin_limit = prm.spin_limit > 0 ? prm.spin_limit : kDefaultSpinLimit;
+    COLAGB_CUDA(cudaMemsetAsync(s.counters, 0, 8 * sizeof(unsigned int), st));
+    bool ran = false;
+    COLAGB_TRY((cg_dense_solve<T, S>(d, st, &ran)));
+    if (ran) return finish_fused(s, res, st);
+  }
+  FusedArgs<T, S> a;
   a.kind = leaf->kind;
   a.vals = static_cast<const S*>(leaf->data);
   a.lda = leaf->ld;
