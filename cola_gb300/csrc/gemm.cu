@@ -385,13 +385,14 @@ static int launch_tile(GemmArgs<T, S>& g, int split, bool xk, cudaStream_t st) {
   return launch_form<T, S, BM, BN, BK, WM, WN, WK, 2, false, false>(g, st);
 }
 
-// Tile choice.  Short products with many columns (Kronecker factors; K <= 256): 128 columns wide, one
-// warp group, 48 or 64 rows, whichever pads M less.  Otherwise 64 x 64 while that gives every SM a
-// tile, then the column tile that N fills.  Split: clusters along k until the grid covers 1.5 times the
-// SMs, each CTA keeping at least two k-slices.  Measured (FP32, back-to-back launches, which cost 6.2 us
-// for the smallest product): 4096 x 4096 x 32 35 us (64 x 32, split 4; 39 us for 64 x 64 tiles), x 512
-// 370 us = 46 TFLOP/s; 1500 x 1500 x 16 8.4 us (split 8; 10.3 us at split 4); 3000 x 3000 x 8 14.5 us;
-// 48 x 48 x 36,864 12.3 us (16.5 us in 64-row tiles, 24.7 us in 16 x 16 ones).
+// Tile choice.  Short FP32 sums (K <= 256: Kronecker factors above all) keep the plain order of k, one
+// warp group and no split: 48 or 64 rows x 128 columns, whichever pads M less, while that gives every SM a
+// tile, else 32 x 32 (32 x 16 for few columns).  Longer sums: 64 x 64 while that gives every SM a tile, else
+// the column tile that N fills, with clusters along k until the grid covers 1.5 times the SMs and each
+// CTA keeps at least two k-slices.  Measured (FP32, back-to-back launches, which cost 6.2 us for the
+// smallest product): 4096 x 4096 x 32 35 us (64 x 32, split 4; 39 us for 64 x 64 tiles), x 512 370 us = 46
+// TFLOP/s; 1500 x 1500 x 16 8.4 us (split 8; 10.3 us at split 4); 3000 x 3000 x 8 14.5 us; 48 x 48 x 36,864
+// 12.4 us (16.5 us in 64-row tiles); 128 x 128 x 2048 8.2 us; 64 x 64 x 262,144 84 us.
 template <class T, class S>
 int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, int64_t x_p, int64_t x_k, T* Y,
                    int64_t y_p, int64_t y_m, int64_t P, int64_t q, T alpha, T beta, const int* skip,
@@ -418,10 +419,12 @@ int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, in
     return s;
   };
   if constexpr (std::is_same<T, float>::value) {
-    if (g.N > 64 && K <= 256) {
+    if (K <= 256) {
       const bool b48 = ceil_div(M, 48) * 48 < ceil_div(M, 64) * 64;
       if (b48 && tiles(48, 128) >= sms) return launch_tile<T, S, 48, 128, 16, 2, 2, 1, 3>(g, 1, xk, st);
       if (!b48 && tiles(64, 128) >= sms) return launch_tile<T, S, 64, 128, 16, 2, 2, 1, 3>(g, 1, xk, st);
+      if (g.N > 16) return launch_tile<T, S, 32, 32, 32, 2, 2, 1, 3>(g, 1, xk, st);
+      return launch_tile<T, S, 32, 16, 32, 2, 1, 1, 4>(g, 1, xk, st);
     }
     if (g.N > 32 && (tiles(64, 64) >= sms || (g.N <= 64 && K >= 512)))
       return launch_tile<T, S, 64, 64, 32, 2, 1, 2, 3>(g, split_for(64, 64, 32), xk, st);

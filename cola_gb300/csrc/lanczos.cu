@@ -224,22 +224,39 @@ __global__ void __launch_bounds__(256) k_lz_norm(const T* v, int64_t n, int64_t 
   }
 }
 
-template <class T>
+// VEC = 4: FP32 blocks of 4, 8, ... columns or a single one with n % 4 == 0, 16-byte aligned.
+template <class T, int VEC>
 __global__ void k_lz_scale(T* v, int64_t n, int64_t bs, LzState<T> s) {
   if (*s.done) return;
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n * bs; u += (int64_t)gridDim.x * blockDim.x)
-    v[u] = v[u] / s.nrm[u % bs];
+  const int64_t units = n * bs / VEC;
+  const unsigned C = VEC == 4 && bs > 1 ? (unsigned)(bs / VEC) : (unsigned)bs;
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned c = bs == 1 ? 0u : units < ((int64_t)1 << 32) ? (unsigned)u % C : (unsigned)(u % C);
+    if constexpr (VEC == 4) {
+      float4* p = reinterpret_cast<float4*>(v) + u;
+      float4 x = *p;
+      if (bs == 1) {
+        const float d = s.nrm[0];
+        x.x /= d; x.y /= d; x.z /= d; x.w /= d;
+      } else {
+        const float4 d = reinterpret_cast<const float4*>(s.nrm)[c];
+        x.x /= d.x; x.y /= d.y; x.z /= d.z; x.w /= d.w;
+      }
+      *p = x;
+    } else {
+      v[u] = v[u] / s.nrm[c];
+    }
+  }
 }
 
 // diag[b][i-1] = <w, V[i]>
-template <class T>
-__global__ void __launch_bounds__(256) k_lz_alpha(const T* w, const T* vi, int64_t n, int64_t bs, T* diag,
-                                                  int max_iters, LzState<T> s) {
+__global__ void __launch_bounds__(256) k_lz_alpha(const float* w, const float* vi, int64_t n, int64_t bs, float* diag,
+                                                  int max_iters, LzState<float> s) {
   if (*s.done) return;
-  __shared__ T smem[256];
-  lz_colsum<T>(n, bs, w, vi, s.npart + (int64_t)blockIdx.x * bs, smem);
+  __shared__ float smem[256];
+  lz_colsum<float>(n, bs, w, vi, s.npart + (int64_t)blockIdx.x * bs, smem);
   if (lz_last_block(s.counters + 1)) {
-    __shared__ T tot[kLzStage], red[32];
+    __shared__ float tot[kLzStage], red[32];
     lz_stage(s.npart, gridDim.x, bs, tot, red, smem);
     const int i = *s.step;
     for (int64_t b = threadIdx.x; b < bs; b += blockDim.x)
@@ -248,145 +265,187 @@ __global__ void __launch_bounds__(256) k_lz_alpha(const T* w, const T* vi, int64
   }
 }
 
-// w -= diag[i-1] V[i] + subdiag[i-1] V[i-1]
-template <class T>
-__global__ void k_lz_three_term(T* w, const T* vi, const T* vim1, int64_t n, int64_t bs, const T* diag,
-                                const T* subdiag, int max_iters, LzState<T> s) {
-  if (*s.done) return;
-  const int i = *s.step;
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n * bs; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = u % bs;
-    w[u] -= diag[b * max_iters + (i - 1)] * vi[u] + subdiag[b * (max_iters + 1) + (i - 1)] * vim1[u];
-  }
+// ---------------------------------------------------------------------------------------------
+// FP32 step after w = A V[i] (bs probes):
+//   k_lz_alpha      diag[i-1] = <w, V[i]>
+//   TERMS_PROJ      w -= diag[i-1] V[i] + subdiag[i-1] V[i-1] as the run is staged, then h1 = V^T w
+//   SUB_PROJ        w -= V h1, then h2 = V^T w on the same run: the second read of a run's slots follows
+//                   the first at once and hits L1 / L2
+//   k_lz_fin        w -= V h2 with |w| per column summed on the way; the last CTA does the bookkeeping
+// and a reduction of the CTAs' partial projections after each projection.  A single FP32 vector's sums
+// decide the last bits of the quadrature, so every sum keeps one fixed order: the partition into runs,
+// the lane and slot-team orders below and the plain order of j for each element of w.  Before, the
+// three-term update, the two subtractions and a second norm of the same vector were sweeps and launches
+// of their own (12 a step beside the operator; now 7), and the reduction read its partials 4 bytes per
+// sector (7.2 us for 40 x 16 sums of 608 partials).
+enum { LZ_TERMS_PROJ = 0, LZ_SUB_PROJ = 1 };
+
+struct LzStep {
+  const float* basis;
+  float* w;                // slot i + 1
+  const float *vi, *vim1;  // slots i, i - 1
+  const float *diag, *subdiag;
+  int64_t n, bs, chunk;    // chunk: rows of a CTA's run
+  int64_t slots;
+  int max_iters;
+  LzState<float> s;
+};
+
+__device__ __forceinline__ float lz_term(float w, float d, float vi, float sb, float vim1) {
+  w -= d * vi + sb * vim1;
+  return w;
 }
 
-// Projection partials: hpart[blk][j][b] = sum over the block's rows of V[j][r][b] * w[r][b], j = 1..i.
-// Each block owns a contiguous row range.  Four basis slots per pass: w is read once for the four,
-// and the four partial sums share one tree reduction (one pass per slot re-read w and waited on a
-// reduction per slot -- this kernel is most of an SLQ run's time).
-template <class T>
-__global__ void __launch_bounds__(256) k_lz_project(const T* basis, const T* w, int64_t n, int64_t bs,
-                                                    int64_t slots, LzState<T> s) {
-  if (*s.done) return;
-  constexpr int JB = 4;
-  __shared__ T smem[JB * 256];
-  const int i = *s.step;
-  const int64_t rows_per_block = ceil_div(n, gridDim.x);
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
-  const int64_t r1 = r0 + rows_per_block < n ? r0 + rows_per_block : n;
-  T* out = s.hpart + (int64_t)blockIdx.x * slots * bs;
-  const int t = threadIdx.x;
-  const int64_t slot = n * bs;
-  for (int64_t b0 = 0; b0 < bs; b0 += blockDim.x) {
-    const int bc = (int)((bs - b0) < (int64_t)blockDim.x ? (bs - b0) : (int64_t)blockDim.x);
-    const int rpp = blockDim.x / bc;
-    const int my_b = t % bc, my_r = t / bc;
-    for (int j0 = 1; j0 <= i; j0 += JB) {
-      const int nj = (i - j0 + 1) < JB ? (i - j0 + 1) : JB;
-      T acc[JB] = {T(0), T(0), T(0), T(0)};
-      if (my_r < rpp) {
-        const T* v0 = basis + (int64_t)j0 * slot + b0 + my_b;
-        for (int64_t r = r0 + my_r; r < r1; r += rpp) {
-          const T wv = w[r * bs + b0 + my_b];
-#pragma unroll
-          for (int q = 0; q < JB; ++q)
-            if (q < nj) acc[q] += v0[(int64_t)q * slot + r * bs] * wv;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < JB; ++q) smem[q * 256 + t] = acc[q];
-      __syncthreads();
-      for (int wd = rpp; wd > 1;) {  // tree over the row slots, all JB sums at once
-        const int h = (wd + 1) >> 1;
-        if (my_r < wd - h) {
-#pragma unroll
-          for (int q = 0; q < JB; ++q) smem[q * 256 + t] += smem[q * 256 + t + h * bc];
-        }
-        __syncthreads();
-        wd = h;
-      }
-      if (t < bc) {
-        for (int q = 0; q < nj; ++q) out[(int64_t)(j0 + q) * bs + b0 + t] = smem[q * 256 + t];
-      }
-      __syncthreads();
+// sum over j = 1..i, in that order, of V[j] h[j] at one entry / two / four entries (offset o, columns b..)
+__device__ __forceinline__ float lz_comb1(const float* basis, int64_t N, int64_t o, const float* h, int64_t bs, int i) {
+  float acc = 0.f;
+  const float* v = basis + N + o;
+#pragma unroll 16
+  for (int j = 1; j <= i; ++j, v += N) acc += __ldg(v) * __ldg(h + (int64_t)j * bs);
+  return acc;
+}
+__device__ __forceinline__ float2 lz_comb2(const float* basis, int64_t N, int64_t o, const float* h, int i) {
+  float2 acc = make_float2(0.f, 0.f);
+  const float* v = basis + N + o;
+#pragma unroll 16
+  for (int j = 1; j <= i; ++j, v += N) {
+    const float2 x = __ldg(reinterpret_cast<const float2*>(v));
+    const float c = __ldg(h + j);
+    acc.x += x.x * c;
+    acc.y += x.y * c;
+  }
+  return acc;
+}
+__device__ __forceinline__ float4 lz_comb4(const float* basis, int64_t N, int64_t o, const float* h, int64_t bs, int i) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* v = basis + N + o;
+  if (bs == 1) {
+#pragma unroll 12
+    for (int j = 1; j <= i; ++j, v += N) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(v));
+      const float c = __ldg(h + j);
+      acc.x += x.x * c;
+      acc.y += x.y * c;
+      acc.z += x.z * c;
+      acc.w += x.w * c;
+    }
+  } else {
+#pragma unroll 8
+    for (int j = 1; j <= i; ++j, v += N) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(v));
+      const float4 c = __ldg(reinterpret_cast<const float4*>(h + (int64_t)j * bs));
+      acc.x += x.x * c.x;
+      acc.y += x.y * c.y;
+      acc.z += x.z * c.z;
+      acc.w += x.w * c.w;
     }
   }
+  return acc;
 }
 
-// Single-vector form (bs == 1, n % 4 == 0): block blk owns rows [blk * chunk, (blk + 1) * chunk) with
-// chunk a multiple of 128.  w's chunk is staged once in shared memory; warp q takes slots j = 1 + q,
-// 1 + q + nwarps, ...: its lanes stream the slot's chunk with 128-bit loads (all of a slot's loads in
-// flight at once), multiply by w from shared memory and finish with one shuffle reduction per slot.
-// One pass reads each filled slot once, with no block-wide barrier per slot.
-__global__ void __launch_bounds__(256) k_lz_project1(const float* __restrict__ basis, const float* __restrict__ w,
-                                                     int64_t n, int64_t chunk, int64_t slots, LzState<float> s) {
+// Single vector (bs == 1, n % 4 == 0): a CTA's run is `chunk` rows (a multiple of 128); a warp takes whole
+// slots, its lanes stream the run with 128-bit loads against w from shared memory.
+template <int MODE>
+__global__ void __launch_bounds__(512) k_lz_proj1(const __grid_constant__ LzStep a) {
+  const LzState<float>& s = a.s;
   if (*s.done) return;
   extern __shared__ float4 wsm[];
   const int i = *s.step;
-  const int64_t r0 = (int64_t)blockIdx.x * chunk;
-  const int64_t r1 = r0 + chunk < n ? r0 + chunk : n;
-  const int64_t n4 = (r1 - r0) / 4;  // float4 groups in this chunk (n and chunk are multiples of 4)
-  const float4* w4 = reinterpret_cast<const float4*>(w + r0);
-  for (int64_t u = threadIdx.x; u < n4; u += blockDim.x) wsm[u] = w4[u];
+  const int64_t n = a.n, r0 = (int64_t)blockIdx.x * a.chunk;
+  const int64_t r1 = r0 + a.chunk < n ? r0 + a.chunk : n;
+  const int n2 = (int)((r1 - r0) / 2), n4 = n2 / 2;
+  float2* w2 = reinterpret_cast<float2*>(a.w + r0);
+  const float d = MODE == LZ_TERMS_PROJ ? a.diag[i - 1] : 0.f, sb = MODE == LZ_TERMS_PROJ ? a.subdiag[i - 1] : 0.f;
+  for (int u = threadIdx.x; u < n2; u += blockDim.x) {
+    float2 x = w2[u];
+    if (MODE == LZ_TERMS_PROJ) {
+      const float2 p = reinterpret_cast<const float2*>(a.vi + r0)[u], q = reinterpret_cast<const float2*>(a.vim1 + r0)[u];
+      x.x = lz_term(x.x, d, p.x, sb, q.x);
+      x.y = lz_term(x.y, d, p.y, sb, q.y);
+    } else {
+      const float2 c = lz_comb2(a.basis, n, r0 + 2 * u, s.hbuf, i);
+      x.x -= c.x;
+      x.y -= c.y;
+    }
+    w2[u] = x;
+    reinterpret_cast<float2*>(wsm)[u] = x;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  float* out = s.hpart + (int64_t)blockIdx.x * slots;
+  float* out = s.hpart + (int64_t)blockIdx.x * a.slots;
   for (int j = 1 + warp; j <= i; j += nw) {
-    const float4* v4 = reinterpret_cast<const float4*>(basis + (int64_t)j * n + r0);
+    const float4* v4 = reinterpret_cast<const float4*>(a.basis + (int64_t)j * n + r0);
     float acc0 = 0.f, acc1 = 0.f;
-    int64_t u = lane;
+    int u = lane;
 #pragma unroll 4
     for (; u + 32 < n4; u += 64) {
-      const float4 a = __ldg(v4 + u), b = __ldg(v4 + u + 32);
+      const float4 p = __ldg(v4 + u), q = __ldg(v4 + u + 32);
       const float4 x = wsm[u], y = wsm[u + 32];
-      acc0 += a.x * x.x + a.y * x.y + a.z * x.z + a.w * x.w;
-      acc1 += b.x * y.x + b.y * y.y + b.z * y.z + b.w * y.w;
+      acc0 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
+      acc1 += q.x * y.x + q.y * y.y + q.z * y.z + q.w * y.w;
     }
     for (; u < n4; u += 32) {
-      const float4 a = __ldg(v4 + u);
+      const float4 p = __ldg(v4 + u);
       const float4 x = wsm[u];
-      acc0 += a.x * x.x + a.y * x.y + a.z * x.z + a.w * x.w;
+      acc0 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
     }
     const float t = warp_sum(acc0 + acc1);
     if (lane == 0) out[j] = t;
   }
 }
 
-// Block form (bs in {4, 8, 16, 32, 64, 128}, FP32): block blk owns rows [blk * chunk, ...), i.e. one
-// contiguous run of chunk * bs floats per slot.  w's run is staged in shared memory; warp q takes
-// slots j = 1 + q, 1 + q + nwarps, ...; a warp step covers 128 consecutive floats, so lane l always
-// holds column quad l % (bs / 4) and accumulates it in a float4; a shuffle tree over the lanes of
-// the same quad finishes the slot.  128-bit streams, no block-wide barrier per slot.
-__global__ void __launch_bounds__(512) k_lz_projectq(const float* __restrict__ basis, const float* __restrict__ w,
-                                                     int64_t n, int64_t bs, int64_t chunk, int64_t slots,
-                                                     LzState<float> s) {
+// Block form (bs in {4, 8, ..., 128}): a run is chunk * bs contiguous floats per slot, a whole number of
+// 128-float warp steps, so lane l always holds column quad l % (bs / 4).
+template <int MODE>
+__global__ void __launch_bounds__(512) k_lz_projq(const __grid_constant__ LzStep a) {
+  const LzState<float>& s = a.s;
   if (*s.done) return;
   extern __shared__ float4 wsm[];
   const int i = *s.step;
-  const int64_t r0 = (int64_t)blockIdx.x * chunk;
-  const int64_t r1 = r0 + chunk < n ? r0 + chunk : n;
-  const int64_t n4 = (r1 - r0) * bs / 4;  // float4 units of this block's run
-  const float4* w4 = reinterpret_cast<const float4*>(w + r0 * bs);
-  for (int64_t u = threadIdx.x; u < n4; u += blockDim.x) wsm[u] = w4[u];
+  const int64_t n = a.n, bs = a.bs, N = n * bs, r0 = (int64_t)blockIdx.x * a.chunk;
+  const int64_t r1 = r0 + a.chunk < n ? r0 + a.chunk : n;
+  const int n4 = (int)((r1 - r0) * bs / 4), qd = (int)(bs / 4);  // qd: a power of two in [1, 32]
+  float4* w4 = reinterpret_cast<float4*>(a.w + r0 * bs);
+  for (int u = threadIdx.x; u < n4; u += blockDim.x) {
+    float4 x = w4[u];
+    const int b = 4 * (u & (qd - 1));
+    if (MODE == LZ_TERMS_PROJ) {
+      const float4 p = reinterpret_cast<const float4*>(a.vi + r0 * bs)[u], q = reinterpret_cast<const float4*>(a.vim1 + r0 * bs)[u];
+      const float* dg = a.diag + (int64_t)b * a.max_iters + (i - 1);
+      const float* sb = a.subdiag + (int64_t)b * (a.max_iters + 1) + (i - 1);
+      const int64_t m = a.max_iters;
+      x.x = lz_term(x.x, __ldg(dg), p.x, __ldg(sb), q.x);
+      x.y = lz_term(x.y, __ldg(dg + m), p.y, __ldg(sb + (m + 1)), q.y);
+      x.z = lz_term(x.z, __ldg(dg + 2 * m), p.z, __ldg(sb + 2 * (m + 1)), q.z);
+      x.w = lz_term(x.w, __ldg(dg + 3 * m), p.w, __ldg(sb + 3 * (m + 1)), q.w);
+    } else {
+      const float4 c = lz_comb4(a.basis, N, r0 * bs + 4 * u, s.hbuf + b, bs, i);
+      x.x -= c.x;
+      x.y -= c.y;
+      x.z -= c.z;
+      x.w -= c.w;
+    }
+    w4[u] = x;
+    wsm[u] = x;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int qd = (int)(bs / 4);  // column quads per row: a power of two in [1, 32]
-  float* out = s.hpart + (int64_t)blockIdx.x * slots * bs;
+  float* out = s.hpart + (int64_t)blockIdx.x * a.slots * bs;
   for (int j = 1 + warp; j <= i; j += nw) {
-    const float4* v4 = reinterpret_cast<const float4*>(basis + (int64_t)j * n * bs + r0 * bs);
+    const float4* v4 = reinterpret_cast<const float4*>(a.basis + (int64_t)j * N + r0 * bs);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    int64_t u = lane;
+    int u = lane;
 #pragma unroll 4
     for (; u + 32 < n4; u += 64) {
-      const float4 a = __ldg(v4 + u), b = __ldg(v4 + u + 32);
+      const float4 p = __ldg(v4 + u), q = __ldg(v4 + u + 32);
       const float4 x = wsm[u], y = wsm[u + 32];
-      acc.x += a.x * x.x; acc.y += a.y * x.y; acc.z += a.z * x.z; acc.w += a.w * x.w;
-      acc2.x += b.x * y.x; acc2.y += b.y * y.y; acc2.z += b.z * y.z; acc2.w += b.w * y.w;
+      acc.x += p.x * x.x; acc.y += p.y * x.y; acc.z += p.z * x.z; acc.w += p.w * x.w;
+      acc2.x += q.x * y.x; acc2.y += q.y * y.y; acc2.z += q.z * y.z; acc2.w += q.w * y.w;
     }
     for (; u < n4; u += 32) {
-      const float4 a = __ldg(v4 + u);
+      const float4 p = __ldg(v4 + u);
       const float4 x = wsm[u];
-      acc.x += a.x * x.x; acc.y += a.y * x.y; acc.z += a.z * x.z; acc.w += a.w * x.w;
+      acc.x += p.x * x.x; acc.y += p.y * x.y; acc.z += p.z * x.z; acc.w += p.w * x.w;
     }
     acc.x += acc2.x; acc.y += acc2.y; acc.z += acc2.z; acc.w += acc2.w;
     for (int o = 16; o >= qd; o >>= 1) {
@@ -399,114 +458,579 @@ __global__ void __launch_bounds__(512) k_lz_projectq(const float* __restrict__ b
   }
 }
 
-// h[j][b] = sum over blocks of hpart  (one warp per (j, b): lanes take strided blocks, then a
-// shuffle tree; a thread per (j, b) would wait on nblk dependent loads)
-template <class T>
-__global__ void k_lz_reduce_h(int nblk, int64_t bs, int64_t slots, LzState<T> s) {
+// Any bs: a run is `chunk` rows.  Teams of 256 threads take four slots at a time (team q the groups q,
+// q + 4, ...); in a team, threads are rows x columns, w is read once for the four slots and the four
+// sums share one tree over the rows.
+constexpr int kLzTeams = 4;
+template <int MODE>
+__global__ void __launch_bounds__(256 * kLzTeams) k_lz_projx(const __grid_constant__ LzStep a) {
+  const LzState<float>& s = a.s;
   if (*s.done) return;
+  constexpr int JB = 4, TT = 256;
+  __shared__ float smem_all[kLzTeams * JB * TT];
+  const int i = *s.step;
+  const int64_t n = a.n, bs = a.bs, N = n * bs;
+  const int64_t r0 = (int64_t)blockIdx.x * a.chunk < n ? (int64_t)blockIdx.x * a.chunk : n;
+  const int64_t r1 = r0 + a.chunk < n ? r0 + a.chunk : n;
+  float* const w = a.w;
+  for (int64_t u = r0 * bs + threadIdx.x; u < r1 * bs; u += blockDim.x) {
+    const int64_t b = u % bs;
+    if (MODE == LZ_TERMS_PROJ)
+      w[u] = lz_term(w[u], a.diag[b * a.max_iters + (i - 1)], a.vi[u], a.subdiag[b * (a.max_iters + 1) + (i - 1)], a.vim1[u]);
+    else
+      w[u] -= lz_comb1(a.basis, N, u, s.hbuf + b, bs, i);
+  }
+  __syncthreads();
+  const int team = threadIdx.x / TT, t = threadIdx.x % TT;
+  float* const smem = smem_all + team * JB * TT;
+  auto team_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(team + 1) : "memory"); };
+  float* out = s.hpart + (int64_t)blockIdx.x * a.slots * bs;
+  for (int64_t b0 = 0; b0 < bs; b0 += TT) {
+    const int bc = (int)((bs - b0) < TT ? (bs - b0) : TT);
+    const int rpp = TT / bc;
+    const int my_b = t % bc, my_r = t / bc;
+    for (int j0 = 1 + JB * team; j0 <= i; j0 += JB * kLzTeams) {
+      const int nj = (i - j0 + 1) < JB ? (i - j0 + 1) : JB;
+      float acc[JB] = {0.f, 0.f, 0.f, 0.f};
+      if (my_r < rpp) {
+        const float* v0 = a.basis + (int64_t)j0 * N + b0 + my_b;
+        for (int64_t r = r0 + my_r; r < r1; r += rpp) {
+          const float wv = w[r * bs + b0 + my_b];
+#pragma unroll
+          for (int q = 0; q < JB; ++q)
+            if (q < nj) acc[q] += v0[(int64_t)q * N + r * bs] * wv;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < JB; ++q) smem[q * TT + t] = acc[q];
+      team_sync();
+      for (int wd = rpp; wd > 1;) {  // tree over the row slots, all JB sums at once
+        const int h = (wd + 1) >> 1;
+        if (my_r < wd - h) {
+#pragma unroll
+          for (int q = 0; q < JB; ++q) smem[q * TT + t] += smem[q * TT + t + h * bc];
+        }
+        team_sync();
+        wd = h;
+      }
+      if (t < bc) {
+        for (int q = 0; q < nj; ++q) out[(int64_t)(j0 + q) * bs + b0 + t] = smem[q * TT + t];
+      }
+      team_sync();
+    }
+  }
+}
+
+// h[j][b] = sum over the CTAs of hpart: 32 interleaved sums, then a tree over them.  32 neighbouring (j, b)
+// per CTA so that the partials are read by whole sectors.
+__global__ void __launch_bounds__(1024) k_lz_reduce32(int nblk, int64_t bs, int64_t slots, LzState<float> s) {
+  if (*s.done) return;
+  __shared__ float part[32][33];
   const int i = *s.step;
   const int64_t total = (int64_t)(i + 1) * bs;
-  const int lane = threadIdx.x & 31;
-  const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t u = warp0; u < total; u += nwarps) {
-    T acc = T(0);
-    if (u >= bs)  // slot 0 is the zero vector
-      for (int q = lane; q < nblk; q += 32) acc += s.hpart[(int64_t)q * slots * bs + u];
-    acc = warp_sum(acc);
-    if (lane == 0) s.hbuf[u] = acc;
+  const int l = threadIdx.x & 31, q0 = threadIdx.x >> 5;
+  for (int64_t u0 = (int64_t)blockIdx.x * 32; u0 < total; u0 += (int64_t)gridDim.x * 32) {
+    float acc = 0.f;
+    const int64_t u = u0 + l;
+    if (u < total && u >= bs)  // slot 0 is the zero vector
+#pragma unroll 4
+      for (int q = q0; q < nblk; q += 32) acc += __ldg(s.hpart + (int64_t)q * slots * bs + u);
+    part[q0][l] = acc;
+    __syncthreads();
+    const float h = warp_sum(part[l][q0]);
+    if (l == 0 && u0 + q0 < total) s.hbuf[u0 + q0] = h;
+    __syncthreads();
   }
 }
 
-// w -= sum_j V[j] h[j]  (128-bit accesses for FP32 when bs is a multiple of 4)
-template <class T>
-__global__ void k_lz_subtract(const T* basis, T* w, int64_t n, int64_t bs, LzState<T> s) {
+// The last subtraction with the sums of squares of lz_colsum on the way (the same rows per thread), then
+// subdiag[b][i] = |w|, i += 1 and the stop test of lanczos_fact.cond_fun in the last CTA.
+__global__ void __launch_bounds__(256) k_lz_fin(const __grid_constant__ LzStep a, float* subdiag, double tol) {
+  const LzState<float>& s = a.s;
   if (*s.done) return;
-  const int i = *s.step;
-  if constexpr (std::is_same<T, float>::value) {
-    if (bs == 1 && n % 4 == 0) {  // one coefficient per slot, four rows per 128-bit access
-      const int64_t n4 = n / 4;
-      float4* w4 = reinterpret_cast<float4*>(w);
-      for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n4; u += (int64_t)gridDim.x * blockDim.x) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int j = 1; j <= i; ++j) {
-          const float4 v = __ldg(reinterpret_cast<const float4*>(basis + (int64_t)j * n) + u);
-          const float h = s.hbuf[j];
-          acc.x += v.x * h;
-          acc.y += v.y * h;
-          acc.z += v.z * h;
-          acc.w += v.w * h;
-        }
-        float4 wv = w4[u];
-        wv.x -= acc.x;
-        wv.y -= acc.y;
-        wv.z -= acc.z;
-        wv.w -= acc.w;
-        w4[u] = wv;
+  __shared__ float4 smem4[256];
+  float* const smem = reinterpret_cast<float*>(smem4);
+  const int i = *s.step, t = threadIdx.x;
+  const int64_t n = a.n, bs = a.bs, N = n * bs;
+  float* const out = s.npart + (int64_t)blockIdx.x * bs;
+  const bool al = (reinterpret_cast<uintptr_t>(a.basis) % 16) == 0 && (reinterpret_cast<uintptr_t>(a.w) % 16) == 0;
+  const bool one = bs == 1 && n % 4 == 0;
+  if (al && (one || (bs % 4 == 0 && bs <= 1024))) {
+    const int64_t rows = one ? n / 4 : n;  // a single column: rows of four entries
+    const int qd = one ? 1 : (int)(bs / 4), rpp = 256 / qd;
+    const int my_q = t % qd, my_r = t / qd;
+    float4 acc[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto term = [&](int64_t r, float4& d) {
+      const int64_t o = (r * qd + my_q) * 4;
+      float4 x = *reinterpret_cast<const float4*>(a.w + o);
+      const float4 c = lz_comb4(a.basis, N, o, s.hbuf + (one ? 0 : 4 * my_q), bs, i);
+      x.x -= c.x;
+      x.y -= c.y;
+      x.z -= c.z;
+      x.w -= c.w;
+      *reinterpret_cast<float4*>(a.w + o) = x;
+      d.x += x.x * x.x;
+      d.y += x.y * x.y;
+      d.z += x.z * x.z;
+      d.w += x.w * x.w;
+    };
+    if (my_r < rpp) {
+      const int64_t stride = (int64_t)rpp * gridDim.x;
+      int64_t r = (int64_t)blockIdx.x * rpp + my_r;
+      for (; r + 3 * stride < rows; r += 4 * stride) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) term(r + u * stride, acc[u]);
       }
-      return;
+      for (; r < rows; r += stride) term(r, acc[0]);
     }
-    if (bs % 4 == 0) {
-      const int64_t n4 = n * bs / 4;
-      float4* w4 = reinterpret_cast<float4*>(w);
-      for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n4; u += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = (4 * u) % bs;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int j = 1; j <= i; ++j) {
-          const float4 v = reinterpret_cast<const float4*>(basis + (int64_t)j * n * bs)[u];
-          const float* h = s.hbuf + (int64_t)j * bs + b;
-          acc.x += v.x * h[0];
-          acc.y += v.y * h[1];
-          acc.z += v.z * h[2];
-          acc.w += v.w * h[3];
-        }
-        float4 wv = w4[u];
-        wv.x -= acc.x;
-        wv.y -= acc.y;
-        wv.z -= acc.z;
-        wv.w -= acc.w;
-        w4[u] = wv;
+    float4 tot;
+    tot.x = (acc[0].x + acc[1].x) + (acc[2].x + acc[3].x);
+    tot.y = (acc[0].y + acc[1].y) + (acc[2].y + acc[3].y);
+    tot.z = (acc[0].z + acc[1].z) + (acc[2].z + acc[3].z);
+    tot.w = (acc[0].w + acc[1].w) + (acc[2].w + acc[3].w);
+    smem4[t] = tot;
+    __syncthreads();
+    for (int w = rpp; w > 1;) {
+      const int h = (w + 1) >> 1;
+      if (my_r < w - h) {
+        const float4 o = smem4[t + h * qd];
+        smem4[t].x += o.x;
+        smem4[t].y += o.y;
+        smem4[t].z += o.z;
+        smem4[t].w += o.w;
       }
-      return;
+      __syncthreads();
+      w = h;
     }
+    if (one) {
+      if (t == 0) out[0] = (smem4[0].x + smem4[0].y) + (smem4[0].z + smem4[0].w);
+    } else if (t < qd) {
+      reinterpret_cast<float4*>(out)[t] = smem4[t];
+    }
+    __syncthreads();
+  } else {
+    lz_partials<float>(n, bs,
+                       [&](int64_t r, int64_t b) {
+                         const int64_t o = r * bs + b;
+                         const float x = a.w[o] - lz_comb1(a.basis, N, o, s.hbuf + b, bs, i);
+                         a.w[o] = x;
+                         return x * x;
+                       },
+                       out, smem);
   }
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n * bs; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = u % bs;
-    T acc = T(0);
-    for (int j = 1; j <= i; ++j) acc += basis[(int64_t)j * n * bs + u] * s.hbuf[(int64_t)j * bs + b];
-    w[u] -= acc;
-  }
-}
-
-// subdiag[b][i] = |w| ; i += 1 ; stop test of lanczos_fact.cond_fun
-template <class T>
-__global__ void __launch_bounds__(256) k_lz_finish(const T* w, int64_t n, int64_t bs, T* subdiag, int max_iters,
-                                                   double tol, LzState<T> s) {
-  if (*s.done) return;
-  __shared__ T smem[256];
-  lz_colsum<T>(n, bs, w, w, s.npart + (int64_t)blockIdx.x * bs, smem);
   if (lz_last_block(s.counters + 2)) {
     __shared__ int s_any;
-    __shared__ T tot[kLzStage], red[32];
+    __shared__ float tot[kLzStage], red[32];
     lz_stage(s.npart, gridDim.x, bs, tot, red, smem);
-    const int i = *s.step;
-    if (threadIdx.x == 0) s_any = 0;
+    if (t == 0) s_any = 0;
     __syncthreads();
-    for (int64_t b = threadIdx.x; b < bs; b += blockDim.x) {
-      const T nv = sqrt(lz_total(s.npart, gridDim.x, bs, b, tot));
-      subdiag[b * (max_iters + 1) + i] = nv;
-      const T first = subdiag[b * (max_iters + 1) + 1];
-      if (nv > (T)tol * first) atomicOr(&s_any, 1);
+    for (int64_t b = t; b < bs; b += blockDim.x) {
+      const float nv = sqrt(lz_total(s.npart, gridDim.x, bs, b, tot));
+      s.nrm[b] = nv;  // what V[i + 1] is divided by
+      subdiag[b * (a.max_iters + 1) + i] = nv;
+      const float first = subdiag[b * (a.max_iters + 1) + 1];
+      if (nv > (float)tol * first) atomicOr(&s_any, 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (t == 0) {
       const int ni = i + 1;
       *s.step = ni;
-      *s.done = !(ni <= max_iters && (s_any || ni <= 1));
+      *s.done = !(ni <= a.max_iters && (s_any || ni <= 1));
       s.counters[2] = 0;
     }
   }
+}
+
+// Which projection form a run of the FP32 method uses, and its launch shape (nb: the partials' capacity).
+struct LzForm {
+  int form = 2;  // 0: k_lz_proj1, 1: k_lz_projq, 2: k_lz_projx
+  int blocks = 1;
+  int64_t chunk = 0;
+  size_t smem = 0;
+};
+static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, LzForm& f) {
+  const bool al = (uintptr_t)basis % 16 == 0;
+  f.blocks = nb;
+  f.chunk = ceil_div(n, (int64_t)nb);
+  int64_t step = 0;
+  if (bs == 1 && n % 4 == 0 && al) step = 128;
+  else if (bs >= 4 && bs <= 128 && (bs & (bs - 1)) == 0 && al) step = 128 / bs;
+  if (step == 0) return COLAGB_OK;
+  const int64_t chunk = ceil_div(f.chunk, step) * step;  // a whole number of 128-float warp steps
+  const size_t smem = (size_t)(chunk * bs) * sizeof(float);
+  if (smem > 160 * 1024) return COLAGB_OK;
+  f.form = bs == 1 ? 0 : 1;
+  f.chunk = chunk;
+  f.blocks = (int)ceil_div(n, chunk);
+  f.smem = smem;
+  if (f.form == 0) {
+    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_proj1<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_proj1<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  } else {
+    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_projq<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_projq<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  }
+  return COLAGB_OK;
+}
+
+template <int MODE>
+static void lz_project(const LzForm& f, const LzStep& a, cudaStream_t st) {
+  if (f.form == 0) k_lz_proj1<MODE><<<f.blocks, 512, f.smem, st>>>(a);
+  else if (f.form == 1) k_lz_projq<MODE><<<f.blocks, 512, f.smem, st>>>(a);
+  else k_lz_projx<MODE><<<f.blocks, 256 * kLzTeams, 0, st>>>(a);
+}
+
+// Everything of a step after the operator's product, w = slot i + 1 holding A V[i].
+static int lz_step_f32(const LzForm& f, const LzStep& a, int i, int nb, float* diag, float* subdiag, double tol,
+                       cudaStream_t st) {
+  const unsigned rb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * a.bs, 32), 4096));
+  k_lz_alpha<<<nb, 256, 0, st>>>(a.w, a.vi, a.n, a.bs, diag, a.max_iters, a.s);
+  lz_project<LZ_TERMS_PROJ>(f, a, st);
+  k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
+  lz_project<LZ_SUB_PROJ>(f, a, st);
+  k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
+  k_lz_fin<<<nb, 256, 0, st>>>(a, subdiag, tol);
+  return COLAGB_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// FP64 and Arnoldi: one step's orthogonalisation.  w = A V[i] is projected on slots 1..i and the projections removed,
+// twice ("twice is enough"): h = V^T w, w -= V h.  The first pass's h_i is diag[i-1] = <w, V[i]>, and
+// since the pass removes it together with the component on V[i-1], the reference's separate
+// three-term update (lanczos.py:262-266) needs no sweep of its own.
+//
+// Three launches over the filled slots (k_lz_gs), a small reduction after the first two:
+//   PROJECT    h1 = V^T w                        every slot read once
+//   SUB_PROJ   w -= V h1, then h2 = V^T w        each CTA on its own run of rows: the second read of a
+//                                                run's slots follows the first at once and hits L1 / L2
+//   SUB_NORM   w -= V h2, |w| per column, and in the last CTA the step's bookkeeping
+// A CTA owns contiguous runs of whole rows; w's run is staged in shared memory.  Subtracting, a thread
+// owns one 16-byte unit (or several threads share it, each with every G-th slot, when the run has fewer
+// units than the CTA has threads); projecting, a warp owns a slot and its lanes keep fixed columns.  The
+// unit is a float4 for FP32 with bs = 1 or a multiple of 4 on 16-byte boundaries, else one entry.
+//
+// It replaced norm, dot, three-term update and four sweeps, 12 launches a step beside the operator, with one
+// dependent load per slot and thread.
+enum { GS_PROJECT = 0, GS_SUB_PROJ = 1, GS_SUB_NORM = 2 };
+constexpr int kGsThreads = 512;
+
+template <class T>
+struct GsArgs {
+  const T* basis;
+  T* w;
+  int64_t N, bs;       // n * bs entries per slot
+  int run;             // entries of a run: whole rows, whole units
+  int64_t slots;
+  T* subdiag;          // SUB_NORM of Lanczos (null for Arnoldi, which only needs |w|)
+  int max_iters;
+  double tol;
+  LzState<T> s;
+};
+
+template <class T, int VEC> struct GsUnit { T v[VEC]; };
+template <class T, int VEC> __device__ __forceinline__ GsUnit<T, VEC> gs_ld(const T* p) {
+  GsUnit<T, VEC> u;
+  if constexpr (VEC == 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    u.v[0] = q.x; u.v[1] = q.y; u.v[2] = q.z; u.v[3] = q.w;
+  } else {
+    u.v[0] = *p;
+  }
+  return u;
+}
+template <class T, int VEC> __device__ __forceinline__ GsUnit<T, VEC> gs_ldg(const T* p) {
+  GsUnit<T, VEC> u;
+  if constexpr (VEC == 4) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+    u.v[0] = q.x; u.v[1] = q.y; u.v[2] = q.z; u.v[3] = q.w;
+  } else {
+    u.v[0] = __ldg(p);
+  }
+  return u;
+}
+template <class T, int VEC> __device__ __forceinline__ void gs_st(T* p, const GsUnit<T, VEC>& u) {
+  if constexpr (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(u.v[0], u.v[1], u.v[2], u.v[3]);
+  else *p = u.v[0];
+}
+
+// Sum over the lanes l, l + C, l + 2C, ... < La of a warp (C columns side by side), result in lanes < C.
+template <class T>
+__device__ __forceinline__ T gs_lane_sum(T x, int C, int La) {
+  if ((C & (C - 1)) == 0) {
+    for (int o = 16; o >= C; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  }
+  T r = x;
+  for (int o = C; o < La; o += C) r += __shfl_sync(0xffffffffu, x, (threadIdx.x & 31) + o);
+  return r;
+}
+
+// STAGED = false: rows too long for shared memory (tens of thousands of columns); w is read back instead.
+template <class T, int VEC, int MODE, bool STAGED>
+__global__ void __launch_bounds__(kGsThreads) k_lz_gs(const __grid_constant__ GsArgs<T> g) {
+  const LzState<T>& s = g.s;
+  if (*s.done) return;
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  T* const red = reinterpret_cast<T*>(gs_smem);  // kGsThreads * VEC
+  T* const stage = red + kGsThreads * VEC;       // the run of w
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  constexpr int NW = kGsThreads / 32;
+  const int i = *s.step;
+  const int bs = (int)g.bs;
+  const bool one = VEC == 4 && bs == 1;         // four rows of a single column per unit
+  const int C = one ? 1 : bs / VEC;             // units of a row
+  const int Cw = C < 32 ? C : 32, La = 32 / Cw * Cw;
+  const int64_t nruns = ceil_div(g.N, (int64_t)g.run);
+  T* const hp = s.hpart + (int64_t)blockIdx.x * g.slots * bs;
+  if (MODE == GS_SUB_NORM) {
+    for (int b = t; b < bs; b += kGsThreads) s.npart[(int64_t)blockIdx.x * bs + b] = T(0);
+  }
+  for (int64_t r = blockIdx.x; r < nruns; r += gridDim.x) {
+    const int64_t e0 = r * g.run;
+    const int len = (int)(g.N - e0 < g.run ? g.N - e0 : g.run), nu = len / VEC;
+    T* const w = g.w + e0;
+    const T* const v = g.basis + e0;
+    T* const ws = STAGED ? stage : w;
+    if (r != blockIdx.x) __syncthreads();  // the previous run's readers are done with ws
+    if (MODE == GS_PROJECT) {
+      if (STAGED)
+        for (int u = t; u < nu; u += kGsThreads) gs_st<T, VEC>(ws + u * VEC, gs_ld<T, VEC>(w + u * VEC));
+    } else {
+      auto sums = [&](int u, int j0, int dj) {  // sum_j V[j] h[j] of unit u over j = j0, j0 + dj, ...
+        GsUnit<T, VEC> acc;
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) acc.v[c] = T(0);
+        const T* vp = v + (int64_t)j0 * g.N + u * VEC;
+        const T* h = s.hbuf + (int64_t)j0 * bs + (one ? 0 : (u % C) * VEC);
+#pragma unroll 8
+        for (int j = j0; j <= i; j += dj, vp += dj * g.N, h += (int64_t)dj * bs) {
+          const GsUnit<T, VEC> x = gs_ldg<T, VEC>(vp);
+          if (one) {
+            const T hh = __ldg(h);
+#pragma unroll
+            for (int c = 0; c < VEC; ++c) acc.v[c] += x.v[c] * hh;
+          } else {
+            const GsUnit<T, VEC> hh = gs_ldg<T, VEC>(h);
+#pragma unroll
+            for (int c = 0; c < VEC; ++c) acc.v[c] += x.v[c] * hh.v[c];
+          }
+        }
+        return acc;
+      };
+      auto finish = [&](int u, const GsUnit<T, VEC>& acc) {
+        GsUnit<T, VEC> x = gs_ld<T, VEC>(w + u * VEC);
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) x.v[c] -= acc.v[c];
+        gs_st<T, VEC>(w + u * VEC, x);
+        if (STAGED) gs_st<T, VEC>(ws + u * VEC, x);
+      };
+      const int G = kGsThreads / nu < i ? kGsThreads / nu : i;
+      if (G >= 2) {
+        const int u = t % nu, gr = t / nu;
+        GsUnit<T, VEC> acc;
+        if (gr < G) {
+          acc = sums(u, 1 + gr, G);
+          if (gr > 0) gs_st<T, VEC>(red + (gr * nu + u) * VEC, acc);
+        }
+        __syncthreads();
+        if (gr == 0) {
+          for (int q = 1; q < G; ++q) {
+            const GsUnit<T, VEC> o = gs_ld<T, VEC>(red + (q * nu + u) * VEC);
+#pragma unroll
+            for (int c = 0; c < VEC; ++c) acc.v[c] += o.v[c];
+          }
+          finish(u, acc);
+        }
+      } else {
+        for (int u = t; u < nu; u += kGsThreads) finish(u, sums(u, 1, 1));
+      }
+    }
+    __syncthreads();  // ws complete
+    // per-column sums of a slot's run against w's: warp per slot (MODE 0 / 1), or of w's squares with
+    // the warps sharing the run (SUB_NORM)
+    const int j_first = MODE == GS_SUB_NORM ? 0 : 1 + warp, j_last = MODE == GS_SUB_NORM ? 0 : i;
+    for (int j = j_first; j <= j_last; j += NW) {
+      const T* const vj = MODE == GS_SUB_NORM ? ws : v + (int64_t)j * g.N;
+      for (int c0 = 0; c0 < C; c0 += Cw) {  // C > 32: 32 columns of units at a time
+        const int cw = C - c0 < Cw ? C - c0 : Cw;
+        const int step = C <= 32 ? La : C;
+        GsUnit<T, VEC> acc, acc2;
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) acc.v[c] = acc2.v[c] = T(0);
+        if (C <= 32 ? lane < La : lane < cw) {
+          const int first = c0 + lane + (MODE == GS_SUB_NORM ? warp * step : 0);
+          const int stride = MODE == GS_SUB_NORM ? NW * step : step;
+          auto term = [&](int u, GsUnit<T, VEC>& a2) {
+            const GsUnit<T, VEC> x = gs_ld<T, VEC>(ws + u * VEC);
+            GsUnit<T, VEC> y;
+            if (MODE == GS_SUB_NORM) y = x;
+            else y = gs_ldg<T, VEC>(vj + u * VEC);
+#pragma unroll
+            for (int c = 0; c < VEC; ++c) a2.v[c] += x.v[c] * y.v[c];
+          };
+          int u = first;
+#pragma unroll 4
+          for (; u + stride < nu; u += 2 * stride) {
+            term(u, acc);
+            term(u + stride, acc2);
+          }
+          if (u < nu) term(u, acc);
+        }
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) acc.v[c] += acc2.v[c];
+        if (one) {
+          acc.v[0] = (acc.v[0] + acc.v[VEC > 1 ? 1 : 0]) + (acc.v[VEC > 2 ? 2 : 0] + acc.v[VEC > 3 ? 3 : 0]);
+        }
+        const int nc = one ? 1 : VEC;
+#pragma unroll
+        for (int c = 0; c < VEC; ++c)
+          if (c < nc) acc.v[c] = gs_lane_sum<T>(acc.v[c], C <= 32 ? C : 32, C <= 32 ? La : 32);
+        if (lane < cw) {
+#pragma unroll
+          for (int c = 0; c < VEC; ++c)
+            if (c < nc) {
+              const int b = (c0 + lane) * nc + c;
+              if (MODE == GS_SUB_NORM) {
+                red[(warp * Cw + lane) * VEC + c] = acc.v[c];
+              } else {
+                T* o = hp + (int64_t)j * bs + b;
+                *o = r == blockIdx.x ? acc.v[c] : *o + acc.v[c];
+              }
+            }
+        }
+        if (MODE == GS_SUB_NORM) {
+          __syncthreads();
+          for (int q = t; q < cw * nc; q += kGsThreads) {
+            const int l = q / nc, c = q % nc;
+            T sum = T(0);
+            for (int ww = 0; ww < NW; ++ww) sum += red[(ww * Cw + l) * VEC + c];
+            s.npart[(int64_t)blockIdx.x * bs + (c0 + l) * nc + c] += sum;
+          }
+          __syncthreads();
+        }
+      }
+    }
+  }
+  if (MODE == GS_SUB_NORM && lz_last_block(s.counters + 2)) {
+    // subdiag[b][i] = |w| ; i += 1 ; stop test of lanczos_fact.cond_fun
+    __shared__ int s_any;
+    __shared__ T tot[kLzStage], bred[32];
+    lz_stage(s.npart, gridDim.x, g.bs, tot, bred, red);
+    if (t == 0) s_any = 0;
+    __syncthreads();
+    for (int64_t b = t; b < g.bs; b += kGsThreads) {
+      const T nv = sqrt(lz_total(s.npart, gridDim.x, g.bs, b, tot));
+      s.nrm[b] = nv;
+      if (g.subdiag) {
+        g.subdiag[b * (g.max_iters + 1) + i] = nv;
+        const T first = g.subdiag[b * (g.max_iters + 1) + 1];
+        if (nv > (T)g.tol * first) atomicOr(&s_any, 1);
+      }
+    }
+    __syncthreads();
+    if (t == 0) {
+      if (g.subdiag) {
+        const int ni = i + 1;
+        *s.step = ni;
+        *s.done = !(ni <= g.max_iters && (s_any || ni <= 1));
+      }
+      s.counters[2] = 0;
+    }
+  }
+}
+
+// h[j][b] = sum over the CTAs of hpart, 32 neighbouring sums per block and eight threads each.  What
+// becomes of them: diag[b][i-1] = h[i][b] after the first pass of Lanczos, column i - 1 of Arnoldi's H
+// (bs, max_iters + 1, max_iters) collects both passes.
+template <class T>
+__global__ void __launch_bounds__(256) k_lz_reduce_h(int nblk, int64_t bs, int64_t slots, T* diag, T* H, int first,
+                                                     int max_iters, LzState<T> s) {
+  if (*s.done) return;
+  __shared__ T part[8][32];
+  const int i = *s.step;
+  const int64_t total = (int64_t)(i + 1) * bs;
+  const int l = threadIdx.x & 31, q0 = threadIdx.x >> 5;
+  for (int64_t u0 = (int64_t)blockIdx.x * 32; u0 < total; u0 += (int64_t)gridDim.x * 32) {
+    const int64_t u = u0 + l;
+    T acc = T(0);
+    if (u < total && u >= bs) {  // slot 0 is the zero vector
+#pragma unroll 8
+      for (int q = q0; q < nblk; q += 8) acc += __ldg(s.hpart + (int64_t)q * slots * bs + u);
+    }
+    part[q0][l] = acc;
+    __syncthreads();
+    if (q0 == 0 && u < total) {
+      const T h = ((part[0][l] + part[1][l]) + (part[2][l] + part[3][l])) +
+                  ((part[4][l] + part[5][l]) + (part[6][l] + part[7][l]));
+      s.hbuf[u] = h;
+      const int64_t j = u / bs, b = u - j * bs;
+      if (diag && j == i) diag[b * max_iters + (i - 1)] = h;
+      if (H && j >= 1) {
+        T* o = H + (b * (max_iters + 1) + (j - 1)) * max_iters + (i - 1);
+        *o = first ? h : *o + h;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Launch plan of k_lz_gs for one run of the method.
+struct GsPlan {
+  int vec = 1, run = 0, blocks = 1;
+  bool staged = true;
+  size_t smem = 0;
+};
+
+template <class T>
+static GsPlan gs_plan(const T* basis, int64_t n, int64_t bs, int max_blocks) {
+  GsPlan p;
+  const int64_t N = n * bs;
+  if (std::is_same<T, float>::value && (uintptr_t)basis % 16 == 0 && (bs % 4 == 0 || (bs == 1 && n % 4 == 0))) p.vec = 4;
+  const int64_t target = std::min<int64_t>(max_blocks, 2 * (int64_t)num_sms());
+  const int64_t unit = bs == 1 ? 32 * p.vec : bs;  // whole rows; a single column: whole warp loads
+  // at most 48 KB of w per run: two CTAs per SM keep their runs' slots in flight together
+  const int64_t most = std::max<int64_t>(1, (48 * 1024 / (int64_t)sizeof(T)) / unit);
+  const int64_t units = std::min(most, std::max<int64_t>(1, ceil_div(ceil_div(N, target), unit)));
+  p.run = (int)(units * unit);
+  p.blocks = (int)std::min<int64_t>(target, ceil_div(N, (int64_t)p.run));
+  p.smem = (size_t)p.run * sizeof(T) + (size_t)kGsThreads * p.vec * sizeof(T);
+  if (p.smem > 200 * 1024) {
+    p.staged = false;
+    p.vec = 1;
+    p.smem = (size_t)kGsThreads * sizeof(T);
+  }
+  return p;
+}
+
+template <class T, int VEC, int MODE, bool STAGED>
+static int launch_gs_form(const GsPlan& p, const GsArgs<T>& a, cudaStream_t st) {
+  auto* f = k_lz_gs<T, VEC, MODE, STAGED>;
+  if (p.smem > 48 * 1024) COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  f<<<p.blocks, kGsThreads, p.smem, st>>>(a);
+  return COLAGB_OK;
+}
+
+template <class T, int MODE>
+static int launch_gs(const GsPlan& p, const GsArgs<T>& a, cudaStream_t st) {
+  if (!p.staged) return launch_gs_form<T, 1, MODE, false>(p, a, st);
+  if constexpr (std::is_same<T, float>::value)
+    if (p.vec == 4) return launch_gs_form<T, 4, MODE, true>(p, a, st);
+  return launch_gs_form<T, 1, MODE, true>(p, a, st);
+}
+
+// The two passes on w (slots 1..i filled): Lanczos with diag / subdiag, Arnoldi with H.
+template <class T>
+static int gs_step(const GsPlan& p, const T* basis, T* w, int64_t n, int64_t bs, int i, T* diag, T* subdiag, T* H,
+                   int max_iters, double tol, const LzState<T>& s, cudaStream_t st) {
+  GsArgs<T> a{basis, w, n * bs, bs, p.run, (int64_t)max_iters + 2, subdiag, max_iters, tol, s};
+  const unsigned rb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * bs, 32), 4096));
+  COLAGB_TRY((launch_gs<T, GS_PROJECT>(p, a, st)));
+  k_lz_reduce_h<T><<<rb, 256, 0, st>>>(p.blocks, bs, a.slots, diag, H, 1, max_iters, s);
+  COLAGB_TRY((launch_gs<T, GS_SUB_PROJ>(p, a, st)));
+  k_lz_reduce_h<T><<<rb, 256, 0, st>>>(p.blocks, bs, a.slots, (T*)nullptr, H, 0, max_iters, s);
+  return launch_gs<T, GS_SUB_NORM>(p, a, st);
 }
 
 // V[1] = V0 / |V0| (init_lanczos) -- norm partials then scale
@@ -811,13 +1335,20 @@ static LzState<T> lz_carve(Bump& ws, int64_t bs, int32_t max_iters, int nb) {
   return s;
 }
 
+// The slots past `last` read as zero, like slot 0: the steps write slots 1..last only.
+template <class T>
+static int clear_unfilled(T* basis, size_t blk, int last, int m, cudaStream_t st) {
+  if (last < m + 1)
+    COLAGB_CUDA(cudaMemsetAsync(basis + (size_t)(last + 1) * blk, 0, sizeof(T) * blk * (size_t)(m + 1 - last), st));
+  return COLAGB_OK;
+}
+
 template <class T>
 static int lanczos_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, const colagb_lanczos_params& prm,
                      T* basis, T* diag, T* subdiag, int32_t* steps, void* workspace, size_t ws_bytes,
                      cudaStream_t st) {
   const int64_t n = A->nodes[A->root].rows;
   const int m = prm.max_iters;
-  const int64_t slots = (int64_t)m + 2;
   const int nb = lz_blocks(n, bs);
   Bump ws(workspace, ws_bytes);
   LzState<T> s = lz_carve<T>(ws, bs, m, nb);
@@ -828,7 +1359,18 @@ static int lanczos_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
     return fail(COLAGB_ERR_WORKSPACE, "colagb_lanczos: workspace too small (need " + std::to_string(ws.peak) + ")");
   const int eg = (int)std::min<int64_t>(std::max<int64_t>(ceil_div(n * bs, 256), 1), (int64_t)num_sms() * 8);
   const size_t blk = (size_t)n * bs;
-  COLAGB_CUDA(cudaMemsetAsync(basis, 0, sizeof(T) * blk * slots, st));
+  const GsPlan plan = gs_plan<T>(basis, n, bs, nb);
+  LzForm form;
+  if constexpr (std::is_same<T, float>::value) COLAGB_TRY(lz_form(basis, n, bs, nb, form));
+  auto scale = [&](T* v) {
+    if constexpr (std::is_same<T, float>::value)
+      if (plan.vec == 4) {
+        k_lz_scale<T, 4><<<(unsigned)std::min<int64_t>(ceil_div((int64_t)blk, 1024), eg), 256, 0, st>>>(v, n, bs, s);
+        return;
+      }
+    k_lz_scale<T, 1><<<eg, 256, 0, st>>>(v, n, bs, s);
+  };
+  COLAGB_CUDA(cudaMemsetAsync(basis, 0, sizeof(T) * blk, st));  // slot 0: V[0] = 0
   COLAGB_CUDA(cudaMemsetAsync(diag, 0, sizeof(T) * bs * m, st));
   COLAGB_CUDA(cudaMemsetAsync(subdiag, 0, sizeof(T) * bs * (m + 1), st));
   COLAGB_CUDA(cudaMemsetAsync(s.counters, 0, 8 * sizeof(unsigned int), st));
@@ -837,97 +1379,41 @@ static int lanczos_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
   T* v1 = basis + blk;
   k_lz_init_copy<T><<<eg, 256, 0, st>>>(V0, ldv0, v1, n, bs);
   k_lz_norm<T><<<nb, 256, 0, st>>>(v1, n, bs, s);
-  k_lz_scale<T><<<eg, 256, 0, st>>>(v1, n, bs, s);
+  scale(v1);
+  k_lz_norm<T><<<nb, 256, 0, st>>>(v1, n, bs, s);  // the loop divides V[1] by its norm again
   COLAGB_CUDA(cudaGetLastError());
   const int every = prm.check_every > 0 ? prm.check_every : 8;
-  // single-vector FP32 runs project with k_lz_project1 (w's chunk in shared memory, a warp per slot)
-  bool p1 = false;
-  int64_t chunk = 0;
-  int nb1 = nb;
-  bool pq = false;  // bs in {4, ..., 128}: k_lz_projectq
-  if constexpr (std::is_same<T, float>::value) {
-    if (bs == 1 && n % 4 == 0 && (uintptr_t)basis % 16 == 0) {
-      chunk = ceil_div(ceil_div(n, nb), 128) * 128;
-      if (chunk * (int64_t)sizeof(float) <= 160 * 1024) {
-        p1 = true;
-        nb1 = (int)ceil_div(n, chunk);
-        COLAGB_CUDA(cudaFuncSetAttribute(k_lz_project1, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(chunk * sizeof(float))));
-      }
-    } else if (bs >= 4 && bs <= 128 && (bs & (bs - 1)) == 0 && (uintptr_t)basis % 16 == 0) {
-      // rows per block so that a block's run is a whole number of 128-float warp steps
-      const int64_t rstep = 128 / bs;
-      chunk = ceil_div(ceil_div(n, nb), rstep) * rstep;
-      if (chunk * bs * (int64_t)sizeof(float) <= 160 * 1024) {
-        pq = true;
-        nb1 = (int)ceil_div(n, chunk);
-        COLAGB_CUDA(cudaFuncSetAttribute(k_lz_projectq, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(chunk * bs * sizeof(float))));
-      }
-    }
-  }
   int host_step = 1;  // the step index the next launch group starts at (upper bound)
-  int hdone = 0;
+  int hstate[5] = {0, 0, 0, 0, 1};  // done, ..., step
   while (true) {
     for (int q = 0; q < every && host_step <= m; ++q, ++host_step) {
       const int i = host_step;  // kernels read the device step; host_step picks the basis slots
       T* vi = basis + (size_t)i * blk;
-      T* vim1 = basis + (size_t)(i - 1) * blk;
       T* w = basis + (size_t)(i + 1) * blk;
-      k_lz_norm<T><<<nb, 256, 0, st>>>(vi, n, bs, s);
-      k_lz_scale<T><<<eg, 256, 0, st>>>(vi, n, bs, s);
+      scale(vi);  // V[i] /= |V[i]|, the norm left by the step before
       Bump ow(opws, opb > 0 ? opb : 1);
       COLAGB_TRY(op_apply<T>(A, A->root, vi, bs, 0, w, bs, 0, bs, 1, T(1), T(0), ow, s.done, st));
-      k_lz_alpha<T><<<nb, 256, 0, st>>>(w, vi, n, bs, diag, m, s);
-      k_lz_three_term<T><<<eg, 256, 0, st>>>(w, vi, vim1, n, bs, diag, subdiag, m, s);
-      for (int pass = 0; pass < 2; ++pass) {
-        if constexpr (std::is_same<T, float>::value) {
-          if (p1)
-            k_lz_project1<<<nb1, 256, chunk * sizeof(float), st>>>(basis, w, n, chunk, slots, s);
-          else if (pq)
-            k_lz_projectq<<<nb1, 512, chunk * bs * sizeof(float), st>>>(basis, w, n, bs, chunk, slots, s);
-          else
-            k_lz_project<T><<<nb, 256, 0, st>>>(basis, w, n, bs, slots, s);
-        } else {
-          k_lz_project<T><<<nb, 256, 0, st>>>(basis, w, n, bs, slots, s);
-        }
-        k_lz_reduce_h<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * bs, 8), 4096)),
-                           256, 0, st>>>((p1 || pq) ? nb1 : nb, bs, slots, s);
-        k_lz_subtract<T><<<eg, 256, 0, st>>>(basis, w, n, bs, s);
+      if constexpr (std::is_same<T, float>::value) {
+        const LzStep a{basis, w, vi, vi - blk, diag, subdiag, n, bs, form.chunk, (int64_t)m + 2, m, s};
+        COLAGB_TRY(lz_step_f32(form, a, i, nb, diag, subdiag, prm.tol, st));
+      } else {
+        COLAGB_TRY(gs_step<T>(plan, basis, w, n, bs, i, diag, subdiag, nullptr, m, prm.tol, s, st));
       }
-      k_lz_finish<T><<<nb, 256, 0, st>>>(w, n, bs, subdiag, m, prm.tol, s);
       COLAGB_CUDA(cudaGetLastError());
     }
-    COLAGB_CUDA(cudaMemcpyAsync(&hdone, s.done, sizeof(int), cudaMemcpyDeviceToHost, st));
+    COLAGB_CUDA(cudaMemcpyAsync(&hstate[0], s.done, sizeof(int), cudaMemcpyDeviceToHost, st));
+    COLAGB_CUDA(cudaMemcpyAsync(&hstate[4], s.step, sizeof(int), cudaMemcpyDeviceToHost, st));
     COLAGB_CUDA(cudaStreamSynchronize(st));
-    if (hdone || host_step > m) break;
+    if (hstate[0] || host_step > m) break;
   }
-  int dstep = 0;
-  COLAGB_CUDA(cudaMemcpyAsync(&dstep, s.step, sizeof(int), cudaMemcpyDeviceToHost, st));
-  COLAGB_CUDA(cudaStreamSynchronize(st));
-  *steps = dstep;
+  COLAGB_TRY(clear_unfilled<T>(basis, blk, hstate[4], m, st));
+  *steps = hstate[4];
   return COLAGB_OK;
 }
 
 
 // ---- Arnoldi (arnoldi.py:303-334) on the same basis slots: Q[j] lives in slot j + 1 ----------
-// H is (bs, max_iters + 1, max_iters) row-major; column idx = step - 1 collects the projection
-// coefficients of both Gram-Schmidt passes and, below them, |w|.
-template <class T>
-__global__ void k_ar_accum_h(T* H, int64_t bs, int max_iters, int first_pass, LzState<T> s) {
-  if (*s.done) return;
-  const int i = *s.step;  // slots 1..i were projected out: rows 0..i-1 of column i-1
-  const int idx = i - 1;
-  const int64_t total = (int64_t)i * bs;
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = u / bs, b = u % bs;
-    T* h = H + (b * (max_iters + 1) + j) * max_iters + idx;
-    const T c = s.hbuf[(j + 1) * bs + b];
-    *h = first_pass ? c : *h + c;
-  }
-}
-
-// w /= max(|w|, tol / 2)  (the new basis vector; |w| from k_lz_norm)
+// w /= max(|w|, tol / 2)  (the new basis vector; |w| from the second pass)
 template <class T>
 __global__ void k_ar_scale_clip(T* w, int64_t n, int64_t bs, double tol, LzState<T> s) {
   if (*s.done) return;
@@ -966,7 +1452,6 @@ static int arnoldi_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
                      T* basis, T* H, int32_t* steps, void* workspace, size_t ws_bytes, cudaStream_t st) {
   const int64_t n = A->nodes[A->root].rows;
   const int m = prm.max_iters;
-  const int64_t slots = (int64_t)m + 2;
   const int nb = lz_blocks(n, bs);
   Bump ws(workspace, ws_bytes);
   LzState<T> s = lz_carve<T>(ws, bs, m, nb);
@@ -977,14 +1462,15 @@ static int arnoldi_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
     return fail(COLAGB_ERR_WORKSPACE, "colagb_arnoldi: workspace too small (need " + std::to_string(ws.peak) + ")");
   const int eg = (int)std::min<int64_t>(std::max<int64_t>(ceil_div(n * bs, 256), 1), (int64_t)num_sms() * 8);
   const size_t blk = (size_t)n * bs;
-  COLAGB_CUDA(cudaMemsetAsync(basis, 0, sizeof(T) * blk * slots, st));
+  const GsPlan plan = gs_plan<T>(basis, n, bs, nb);
+  COLAGB_CUDA(cudaMemsetAsync(basis, 0, sizeof(T) * blk, st));  // slot 0
   COLAGB_CUDA(cudaMemsetAsync(H, 0, sizeof(T) * bs * (m + 1) * (m > 0 ? m : 1), st));
   COLAGB_CUDA(cudaMemsetAsync(s.counters, 0, 8 * sizeof(unsigned int), st));
   k_lz_set_state<T><<<1, 32, 0, st>>>(s, m);
   T* q0 = basis + blk;  // Q[0] = V0 / |V0|
   k_lz_init_copy<T><<<eg, 256, 0, st>>>(V0, ldv0, q0, n, bs);
   k_lz_norm<T><<<nb, 256, 0, st>>>(q0, n, bs, s);
-  k_lz_scale<T><<<eg, 256, 0, st>>>(q0, n, bs, s);
+  k_lz_scale<T, 1><<<eg, 256, 0, st>>>(q0, n, bs, s);
   COLAGB_CUDA(cudaGetLastError());
   const int every = prm.check_every > 0 ? prm.check_every : 8;
   int host_step = 1;  // slot of Q[idx] for the next step (idx = host_step - 1)
@@ -996,15 +1482,7 @@ static int arnoldi_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
       T* w = basis + (size_t)(i + 1) * blk;
       Bump ow(opws, opb > 0 ? opb : 1);
       COLAGB_TRY(op_apply<T>(A, A->root, qi, bs, 0, w, bs, 0, bs, 1, T(1), T(0), ow, s.done, st));
-      for (int pass = 0; pass < 2; ++pass) {  // classical Gram-Schmidt, twice
-        k_lz_project<T><<<nb, 256, 0, st>>>(basis, w, n, bs, slots, s);
-        k_lz_reduce_h<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * bs, 8), 4096)),
-                           256, 0, st>>>(nb, bs, slots, s);
-        k_ar_accum_h<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)i * bs, 256), 4096)), 256,
-                          0, st>>>(H, bs, m, pass == 0, s);
-        k_lz_subtract<T><<<eg, 256, 0, st>>>(basis, w, n, bs, s);
-      }
-      k_lz_norm<T><<<nb, 256, 0, st>>>(w, n, bs, s);
+      COLAGB_TRY(gs_step<T>(plan, basis, w, n, bs, i, nullptr, nullptr, H, m, prm.tol, s, st));
       k_ar_scale_clip<T><<<eg, 256, 0, st>>>(w, n, bs, prm.tol, s);
       k_ar_finish<T><<<1, 256, 0, st>>>(H, bs, m, prm.tol, s);
       COLAGB_CUDA(cudaGetLastError());
@@ -1016,6 +1494,7 @@ static int arnoldi_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
   int dstep = 0;
   COLAGB_CUDA(cudaMemcpyAsync(&dstep, s.step, sizeof(int), cudaMemcpyDeviceToHost, st));
   COLAGB_CUDA(cudaStreamSynchronize(st));
+  COLAGB_TRY(clear_unfilled<T>(basis, blk, dstep, m, st));
   *steps = dstep - 1;  // Arnoldi steps taken (idx)
   return COLAGB_OK;
 }

@@ -618,7 +618,7 @@ int op_apply(const colagb_op* op, int node, const T* X, int64_t ldx, int64_t bsx
               COLAGB_TRY(tc_contract(a_in, false, 1, pre, c[i], f.data, f.dtype, f.ld, r[i], o, 0, r[i], 1, a_f, b_f,
                                      split, ws, skip, st));
             ws.release(tmark);
-          } else if (op->nodes[ch[i]].kind == COLAGB_OP_DENSE) {
+          } else if (op->nodes[ch[i]].kind == COLAGB_OP_DENSE && (q > 4 || pre >= 16)) {
             // one product over all pre * q columns, read and written in place
             COLAGB_TRY(contract_leaf<T>(op->nodes[ch[i]], in, c[i] * q, q, out, r[i] * q, q, pre, q,
                                         direct ? alpha : T(1), direct ? beta : T(0), skip, st));
