@@ -27,6 +27,7 @@
 #include <string>
 #include <vector>
 
+#include "cg_csr.cuh"
 #include "cg_dense.cuh"
 #include "common.cuh"
 #include "ops.cuh"
@@ -1103,6 +1104,34 @@ static int run_fused(const CgPlan& pl, const T* B, int64_t ldb, T* X, int64_t ld
     COLAGB_CUDA(cudaMemsetAsync(s.counters, 0, 8 * sizeof(unsigned int), st));
     bool ran = false;
     COLAGB_TRY((cg_dense_solve<T, S>(d, st, &ran)));
+    if (ran) return finish_fused(s, res, st);
+  }
+  if (leaf->kind == COLAGB_OP_CSR && pl.k == 1 && pl.n < ((int64_t)1 << 31) - 1) {
+    CsrCgArgs<T, S> d;
+    d.indptr = leaf->indptr;
+    d.indices = leaf->indices;
+    d.vals = static_cast<const S*>(leaf->data);
+    d.n = (int)pl.n;
+    d.shift = (T)pl.ff.shift;
+    d.dinv = PK == 1 ? static_cast<const T*>(pl.pdiag->data) : nullptr;
+    d.B = B;
+    d.ldb = ldb;
+    d.X = X;
+    d.ldx = ldx;
+    d.Z = R;
+    d.P0 = Pv;
+    d.P1 = AP;
+    d.part = s.pA;  // pA, pB, pC are consecutive, at least 2 * SMs entries each: 4 * CTAs <= 6 * SMs
+    d.tol = prm.tol;
+    d.max_iters = prm.max_iters;
+    d.hist = hist;
+    d.iters = s.iters;
+    d.count = s.counters + 4;
+    d.err = reinterpret_cast<int*>(s.counters + 6);
+    d.spin_limit = prm.spin_limit > 0 ? prm.spin_limit : kDefaultSpinLimit;
+    COLAGB_CUDA(cudaMemsetAsync(s.counters, 0, 8 * sizeof(unsigned int), st));
+    bool ran = false;
+    COLAGB_TRY((cg_csr_solve<T, S>(d, leaf->nnz, st, &ran)));
     if (ran) return finish_fused(s, res, st);
   }
   FusedArgs<T, S> a;
