@@ -104,14 +104,22 @@ __device__ __forceinline__ void lz_partials4(int64_t n, int64_t bs, const float*
         acc[u].w += x[u].w * y[u].w;
       }
     }
-    for (; r < n; r += stride) {
-      const int64_t o = r * bs + 4 * my_q;
-      const float4 x = __ldg(reinterpret_cast<const float4*>(a + o)), y = __ldg(reinterpret_cast<const float4*>(c + o));
-      acc[0].x += x.x * y.x;
-      acc[0].y += x.y * y.y;
-      acc[0].z += x.z * y.z;
-      acc[0].w += x.w * y.w;
-    }
+    float4 x[3], y[3];  // the last one to three rows, in order
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (r + u * stride < n) {
+        const int64_t o = (r + u * stride) * bs + 4 * my_q;
+        x[u] = __ldg(reinterpret_cast<const float4*>(a + o));
+        y[u] = __ldg(reinterpret_cast<const float4*>(c + o));
+      }
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (r + u * stride < n) {
+        acc[0].x += x[u].x * y[u].x;
+        acc[0].y += x[u].y * y[u].y;
+        acc[0].z += x[u].z * y[u].z;
+        acc[0].w += x[u].w * y[u].w;
+      }
   }
   float4 tot;
   tot.x = (acc[0].x + acc[1].x) + (acc[2].x + acc[3].x);
@@ -179,8 +187,16 @@ __device__ __forceinline__ void lz_stage(const T* part, int nb, int64_t bs, T* t
     const int G = (int)(blockDim.x / kk);
     const int b = (int)(threadIdx.x % kk), g = (int)(threadIdx.x / kk);
     T acc = T(0);
-#pragma unroll 4
-    for (int q = g; q < nb; q += G) acc += __ldcg(part + (int64_t)q * bs + b);
+    constexpr int B = 16;  // loads in flight
+    for (int q = g; q < nb; q += B * G) {
+      T v[B];
+#pragma unroll
+      for (int e = 0; e < B; ++e)
+        if (q + e * G < nb) v[e] = __ldcg(part + (int64_t)(q + e * G) * bs + b);
+#pragma unroll
+      for (int e = 0; e < B; ++e)
+        if (q + e * G < nb) acc += v[e];
+    }
     scratch[threadIdx.x] = acc;
     __syncthreads();
     if (threadIdx.x < kk) {
@@ -296,48 +312,78 @@ __device__ __forceinline__ float lz_term(float w, float d, float vi, float sb, f
   return w;
 }
 
-// sum over j = 1..i, in that order, of V[j] h[j] at one entry / two / four entries (offset o, columns b..)
+// sum over j = 1..i, in that order, of V[j] h[j] at one / two / four entries (offset o, column(s) of h).  The
+// loads of a batch of slots are issued together, the last batch predicated: a remainder loop would wait
+// for one load at a time (74 us instead of 30 for 20 slots of 1.8M entries).
 __device__ __forceinline__ float lz_comb1(const float* basis, int64_t N, int64_t o, const float* h, int64_t bs, int i) {
+  constexpr int B = 16;
   float acc = 0.f;
   const float* v = basis + N + o;
-#pragma unroll 16
-  for (int j = 1; j <= i; ++j, v += N) acc += __ldg(v) * __ldg(h + (int64_t)j * bs);
+  for (int j = 1; j <= i; j += B, v += B * N) {
+    float x[B], c[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (j + q <= i) {
+        x[q] = __ldg(v + q * N);
+        c[q] = __ldg(h + (int64_t)(j + q) * bs);
+      }
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (j + q <= i) acc += x[q] * c[q];
+  }
   return acc;
 }
 __device__ __forceinline__ float2 lz_comb2(const float* basis, int64_t N, int64_t o, const float* h, int i) {
+  constexpr int B = 16;
   float2 acc = make_float2(0.f, 0.f);
   const float* v = basis + N + o;
-#pragma unroll 16
-  for (int j = 1; j <= i; ++j, v += N) {
-    const float2 x = __ldg(reinterpret_cast<const float2*>(v));
-    const float c = __ldg(h + j);
-    acc.x += x.x * c;
-    acc.y += x.y * c;
+  for (int j = 1; j <= i; j += B, v += B * N) {
+    float2 x[B];
+    float c[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (j + q <= i) {
+        x[q] = __ldg(reinterpret_cast<const float2*>(v + q * N));
+        c[q] = __ldg(h + j + q);
+      }
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (j + q <= i) {
+        acc.x += x[q].x * c[q];
+        acc.y += x[q].y * c[q];
+      }
   }
   return acc;
 }
 __device__ __forceinline__ float4 lz_comb4(const float* basis, int64_t N, int64_t o, const float* h, int64_t bs, int i) {
+  constexpr int B = 8;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* v = basis + N + o;
-  if (bs == 1) {
-#pragma unroll 12
-    for (int j = 1; j <= i; ++j, v += N) {
-      const float4 x = __ldg(reinterpret_cast<const float4*>(v));
-      const float c = __ldg(h + j);
-      acc.x += x.x * c;
-      acc.y += x.y * c;
-      acc.z += x.z * c;
-      acc.w += x.w * c;
-    }
-  } else {
-#pragma unroll 8
-    for (int j = 1; j <= i; ++j, v += N) {
-      const float4 x = __ldg(reinterpret_cast<const float4*>(v));
-      const float4 c = __ldg(reinterpret_cast<const float4*>(h + (int64_t)j * bs));
-      acc.x += x.x * c.x;
-      acc.y += x.y * c.y;
-      acc.z += x.z * c.z;
-      acc.w += x.w * c.w;
+  for (int j = 1; j <= i; j += B, v += B * N) {
+    float4 x[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (j + q <= i) x[q] = __ldg(reinterpret_cast<const float4*>(v + q * N));
+    if (bs == 1) {
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (j + q <= i) {
+          const float c = __ldg(h + j + q);
+          acc.x += x[q].x * c;
+          acc.y += x[q].y * c;
+          acc.z += x[q].z * c;
+          acc.w += x[q].w * c;
+        }
+    } else {
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (j + q <= i) {
+          const float4 c = __ldg(reinterpret_cast<const float4*>(h + (int64_t)(j + q) * bs));
+          acc.x += x[q].x * c.x;
+          acc.y += x[q].y * c.y;
+          acc.z += x[q].z * c.z;
+          acc.w += x[q].w * c.w;
+        }
     }
   }
   return acc;
@@ -346,9 +392,10 @@ __device__ __forceinline__ float4 lz_comb4(const float* basis, int64_t N, int64_
 // Single vector (bs == 1, n % 4 == 0): a CTA's run is `chunk` rows (a multiple of 128); a warp takes whole
 // slots, its lanes stream the run with 128-bit loads against w from shared memory.
 template <int MODE>
-__global__ void __launch_bounds__(512) k_lz_proj1(const __grid_constant__ LzStep a) {
+__global__ void __launch_bounds__(512, 2) k_lz_proj1(const __grid_constant__ LzStep a) {
   const LzState<float>& s = a.s;
   if (*s.done) return;
+  constexpr int B = 8;
   extern __shared__ float4 wsm[];
   const int i = *s.step;
   const int64_t n = a.n, r0 = (int64_t)blockIdx.x * a.chunk;
@@ -375,19 +422,19 @@ __global__ void __launch_bounds__(512) k_lz_proj1(const __grid_constant__ LzStep
   float* out = s.hpart + (int64_t)blockIdx.x * a.slots;
   for (int j = 1 + warp; j <= i; j += nw) {
     const float4* v4 = reinterpret_cast<const float4*>(a.basis + (int64_t)j * n + r0);
-    float acc0 = 0.f, acc1 = 0.f;
-    int u = lane;
-#pragma unroll 4
-    for (; u + 32 < n4; u += 64) {
-      const float4 p = __ldg(v4 + u), q = __ldg(v4 + u + 32);
-      const float4 x = wsm[u], y = wsm[u + 32];
-      acc0 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
-      acc1 += q.x * y.x + q.y * y.y + q.z * y.z + q.w * y.w;
-    }
-    for (; u < n4; u += 32) {
-      const float4 p = __ldg(v4 + u);
-      const float4 x = wsm[u];
-      acc0 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
+    float acc0 = 0.f, acc1 = 0.f;  // even and odd 32-quad pieces
+    for (int u = lane; u < n4; u += 32 * B) {
+      float4 v[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (u + 32 * q < n4) v[q] = __ldg(v4 + u + 32 * q);
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (u + 32 * q < n4) {
+          const float4 p = v[q], x = wsm[u + 32 * q];
+          if (q % 2 == 0) acc0 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
+          else acc1 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
+        }
     }
     const float t = warp_sum(acc0 + acc1);
     if (lane == 0) out[j] = t;
@@ -397,9 +444,10 @@ __global__ void __launch_bounds__(512) k_lz_proj1(const __grid_constant__ LzStep
 // Block form (bs in {4, 8, ..., 128}): a run is chunk * bs contiguous floats per slot, a whole number of
 // 128-float warp steps, so lane l always holds column quad l % (bs / 4).
 template <int MODE>
-__global__ void __launch_bounds__(512) k_lz_projq(const __grid_constant__ LzStep a) {
+__global__ void __launch_bounds__(512, 2) k_lz_projq(const __grid_constant__ LzStep a) {
   const LzState<float>& s = a.s;
   if (*s.done) return;
+  constexpr int B = 8;
   extern __shared__ float4 wsm[];
   const int i = *s.step;
   const int64_t n = a.n, bs = a.bs, N = n * bs, r0 = (int64_t)blockIdx.x * a.chunk;
@@ -434,18 +482,18 @@ __global__ void __launch_bounds__(512) k_lz_projq(const __grid_constant__ LzStep
   for (int j = 1 + warp; j <= i; j += nw) {
     const float4* v4 = reinterpret_cast<const float4*>(a.basis + (int64_t)j * N + r0 * bs);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    int u = lane;
-#pragma unroll 4
-    for (; u + 32 < n4; u += 64) {
-      const float4 p = __ldg(v4 + u), q = __ldg(v4 + u + 32);
-      const float4 x = wsm[u], y = wsm[u + 32];
-      acc.x += p.x * x.x; acc.y += p.y * x.y; acc.z += p.z * x.z; acc.w += p.w * x.w;
-      acc2.x += q.x * y.x; acc2.y += q.y * y.y; acc2.z += q.z * y.z; acc2.w += q.w * y.w;
-    }
-    for (; u < n4; u += 32) {
-      const float4 p = __ldg(v4 + u);
-      const float4 x = wsm[u];
-      acc.x += p.x * x.x; acc.y += p.y * x.y; acc.z += p.z * x.z; acc.w += p.w * x.w;
+    for (int u = lane; u < n4; u += 32 * B) {  // even 32-quad pieces into acc, odd ones into acc2
+      float4 v[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (u + 32 * q < n4) v[q] = __ldg(v4 + u + 32 * q);
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (u + 32 * q < n4) {
+          const float4 p = v[q], x = wsm[u + 32 * q];
+          float4& d = q % 2 == 0 ? acc : acc2;
+          d.x += p.x * x.x; d.y += p.y * x.y; d.z += p.z * x.z; d.w += p.w * x.w;
+        }
     }
     acc.x += acc2.x; acc.y += acc2.y; acc.z += acc2.z; acc.w += acc2.w;
     for (int o = 16; o >= qd; o >>= 1) {
@@ -532,9 +580,18 @@ __global__ void __launch_bounds__(1024) k_lz_reduce32(int nblk, int64_t bs, int6
   for (int64_t u0 = (int64_t)blockIdx.x * 32; u0 < total; u0 += (int64_t)gridDim.x * 32) {
     float acc = 0.f;
     const int64_t u = u0 + l;
-    if (u < total && u >= bs)  // slot 0 is the zero vector
-#pragma unroll 4
-      for (int q = q0; q < nblk; q += 32) acc += __ldg(s.hpart + (int64_t)q * slots * bs + u);
+    if (u < total && u >= bs) {  // slot 0 is the zero vector
+      constexpr int B = 10;      // loads in flight
+      for (int q = q0; q < nblk; q += 32 * B) {
+        float v[B];
+#pragma unroll
+        for (int e = 0; e < B; ++e)
+          if (q + 32 * e < nblk) v[e] = __ldg(s.hpart + (int64_t)(q + 32 * e) * slots * bs + u);
+#pragma unroll
+        for (int e = 0; e < B; ++e)
+          if (q + 32 * e < nblk) acc += v[e];
+      }
+    }
     part[q0][l] = acc;
     __syncthreads();
     const float h = warp_sum(part[l][q0]);
@@ -545,7 +602,7 @@ __global__ void __launch_bounds__(1024) k_lz_reduce32(int nblk, int64_t bs, int6
 
 // The last subtraction with the sums of squares of lz_colsum on the way (the same rows per thread), then
 // subdiag[b][i] = |w|, i += 1 and the stop test of lanczos_fact.cond_fun in the last CTA.
-__global__ void __launch_bounds__(256) k_lz_fin(const __grid_constant__ LzStep a, float* subdiag, double tol) {
+__global__ void __launch_bounds__(256, 4) k_lz_fin(const __grid_constant__ LzStep a, float* subdiag, double tol) {
   const LzState<float>& s = a.s;
   if (*s.done) return;
   __shared__ float4 smem4[256];
@@ -675,10 +732,12 @@ static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, LzForm& f)
   return COLAGB_OK;
 }
 
+// A warp takes whole slots: as many warps (8 to 16) as share i slots evenly.
 template <int MODE>
-static void lz_project(const LzForm& f, const LzStep& a, cudaStream_t st) {
-  if (f.form == 0) k_lz_proj1<MODE><<<f.blocks, 512, f.smem, st>>>(a);
-  else if (f.form == 1) k_lz_projq<MODE><<<f.blocks, 512, f.smem, st>>>(a);
+static void lz_project(const LzForm& f, const LzStep& a, int i, cudaStream_t st) {
+  const int rounds = (i + 15) / 16, warps = std::max(8, (i + rounds - 1) / rounds);
+  if (f.form == 0) k_lz_proj1<MODE><<<f.blocks, 32 * warps, f.smem, st>>>(a);
+  else if (f.form == 1) k_lz_projq<MODE><<<f.blocks, 32 * warps, f.smem, st>>>(a);
   else k_lz_projx<MODE><<<f.blocks, 256 * kLzTeams, 0, st>>>(a);
 }
 
@@ -687,9 +746,9 @@ static int lz_step_f32(const LzForm& f, const LzStep& a, int i, int nb, float* d
                        cudaStream_t st) {
   const unsigned rb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * a.bs, 32), 4096));
   k_lz_alpha<<<nb, 256, 0, st>>>(a.w, a.vi, a.n, a.bs, diag, a.max_iters, a.s);
-  lz_project<LZ_TERMS_PROJ>(f, a, st);
+  lz_project<LZ_TERMS_PROJ>(f, a, i, st);
   k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
-  lz_project<LZ_SUB_PROJ>(f, a, st);
+  lz_project<LZ_SUB_PROJ>(f, a, i, st);
   k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
   k_lz_fin<<<nb, 256, 0, st>>>(a, subdiag, tol);
   return COLAGB_OK;

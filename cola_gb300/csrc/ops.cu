@@ -306,6 +306,24 @@ __global__ void axpby_kernel(const T* __restrict__ X, int64_t ldx, int64_t bsx, 
   }
 }
 
+// The same on contiguous blocks, 16 bytes per access (the division per entry and 4-byte accesses took 9.2 us
+// for 1.8M FP32 entries; X and Y at 16-byte boundaries, total a whole number of units).
+template <class T>
+__global__ void axpby_flat_kernel(const T* __restrict__ X, T* __restrict__ Y, int64_t units, T alpha, T beta,
+                                  const int* skip) {
+  if (skip && *skip) return;
+  constexpr int E = 16 / (int)sizeof(T);
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
+    float4 xq = __ldg(reinterpret_cast<const float4*>(X) + u), yq = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (beta != T(0)) yq = reinterpret_cast<const float4*>(Y)[u];
+    const T* x = reinterpret_cast<const T*>(&xq);
+    T* y = reinterpret_cast<T*>(&yq);
+#pragma unroll
+    for (int e = 0; e < E; ++e) y[e] = combine(x[e], alpha, beta, y + e);
+    reinterpret_cast<float4*>(Y)[u] = yq;
+  }
+}
+
 // xp[b][i][c] = X[b][perm[i]][c]: the input of a permuted Sparse node in its stored order.
 template <class T>
 __global__ void k_perm_gather(const int32_t* __restrict__ perm, int64_t n, const T* __restrict__ X, int64_t ldx,
@@ -334,6 +352,13 @@ template <class T>
 int launch_axpby_b(const T* X, int64_t ldx, int64_t bsx, T* Y, int64_t ldy, int64_t bsy, int64_t rows, int64_t k,
                    int64_t batch, T alpha, T beta, const int* skip, cudaStream_t st) {
   if (rows * k == 0) return COLAGB_OK;
+  constexpr int64_t E = 16 / (int64_t)sizeof(T);
+  if (batch == 1 && ldx == k && ldy == k && rows * k % E == 0 && X != Y &&
+      (reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) % 16 == 0) {
+    axpby_flat_kernel<T><<<elementwise_grid(rows * k / E), 256, 0, st>>>(X, Y, rows * k / E, alpha, beta, skip);
+    COLAGB_CUDA(cudaGetLastError());
+    return COLAGB_OK;
+  }
   dim3 grid(elementwise_grid(rows * k), (unsigned)batch);
   axpby_kernel<T><<<grid, 256, 0, st>>>(X, ldx, bsx, Y, ldy, bsy, rows, k, alpha, beta, skip);
   COLAGB_CUDA(cudaGetLastError());
