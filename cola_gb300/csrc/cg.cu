@@ -1157,8 +1157,7 @@ static int run_fused(const CgPlan& pl, const T* B, int64_t ldb, T* X, int64_t ld
   a.vec4 = leaf->kind == COLAGB_OP_DENSE && (pl.n % 4 == 0) && (leaf->ld % 4 == 0) &&
            ((uintptr_t)leaf->data % 16 == 0) && ((uintptr_t)Pv % 16 == 0);
   a.s = s;
-  a.gb.count = s.counters + 4;
-  a.gb.generation = s.counters + 5;
+  a.gb.arrivals = reinterpret_cast<unsigned long long*>(s.counters + 4);
   a.gb.err = reinterpret_cast<int*>(s.counters + 6);
   a.gb.spin_limit = prm.spin_limit > 0 ? prm.spin_limit : kDefaultSpinLimit;
   const size_t smem = 256 * sizeof(T) + 7 * (size_t)pl.k * sizeof(T) + (size_t)pl.k * sizeof(int);

@@ -873,8 +873,7 @@ extern "C" int colagb_cg_batched_csr_solve(const colagb_batched_csr* A, const do
     a.prec_kind = params->preconditioner;
     a.fallback = params->fallback;
     a.mode = params->mode;
-    a.gb.count = w.bar;
-    a.gb.generation = w.bar + 1;
+    a.gb.arrivals = reinterpret_cast<unsigned long long*>(w.bar);
     a.gb.err = reinterpret_cast<int*>(w.bar + 2);
     a.gb.spin_limit = params->spin_limit > 0 ? params->spin_limit : kDefaultSpinLimit;
     const size_t smem = batched_smem(S);

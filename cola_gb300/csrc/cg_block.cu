@@ -21,7 +21,7 @@
 
 namespace colagb {
 
-constexpr int kBT = 256;        // threads per CTA
+constexpr int kBT = 1024;       // threads per CTA, one CTA per SM
 constexpr int kBMaxK = 128;     // columns per launch (the host splits wider blocks)
 
 struct BlockArgs {
@@ -46,77 +46,76 @@ struct BlockArgs {
   GridBarrier gb;
 };
 
-// Per-thread float4 partials of column quad (threadIdx % q, q a power of two <= 32) -> dst[0..4q) as
-// one fixed-order sum: a shuffle tree over the lanes of a warp that share the quad, then warp by warp.
-__device__ __forceinline__ void block_quad_partials(float4 v, int q, float* dst, float4* red) {
+// Per-thread float4 partials of column quad (threadIdx % q, q a power of two <= 32), NV of them -> dst[v][0..4q)
+// as fixed-order sums: a shuffle tree over the lanes of a warp that share the quad, then warp j adds the
+// warps' sums of quad j.
+template <int NV>
+__device__ __forceinline__ void block_quad_partials(float4 (&v)[NV], int q, float* const (&dst)[NV], float4* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o >= q; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    v.z += __shfl_xor_sync(0xffffffffu, v.z, o);
-    v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
+  constexpr int NW = kBT / 32;
+  auto add = [](float4& x, int o) {
+    x.x += __shfl_xor_sync(0xffffffffu, x.x, o);
+    x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
+    x.z += __shfl_xor_sync(0xffffffffu, x.z, o);
+    x.w += __shfl_xor_sync(0xffffffffu, x.w, o);
+  };
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    for (int o = 16; o >= q; o >>= 1) add(v[k], o);
+    if (lane < q) red[k * kBT + lane * NW + warp] = v[k];  // lane l < q holds the warp's sum for quad l
   }
-  if (lane < q) red[warp * 32 + lane] = v;  // lane l < q now holds the warp's sum for quad l
   __syncthreads();
-  if ((int)threadIdx.x < q) {
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int w = 0; w < kBT / 32; ++w) {
-      const float4 x = red[w * 32 + threadIdx.x];
-      t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
+  if (warp < q) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      float4 t = red[k * kBT + warp * NW + lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) add(t, o);
+      if (lane == 0) reinterpret_cast<float4*>(dst[k])[warp] = t;
     }
-    reinterpret_cast<float4*>(dst)[threadIdx.x] = t;
   }
   __syncthreads();
 }
 
-// Column totals of FP32 partials over all CTAs, fixed order: into smem out[0..ncols).
-__device__ __forceinline__ void grid_totals_f(const float* pf, int nb, int64_t stride, int ncols, float* out,
-                                              float* tmp) {
-  const int c = threadIdx.x & 31, g = threadIdx.x >> 5, ng = kBT / 32;
-  for (int cb = 0; cb < ncols; cb += 32) {
-    const int col = cb + c;
-    float acc = 0.f;
-    if (col < ncols)
-      for (int b = g; b < nb; b += ng) acc += pf[(int64_t)b * stride + col];
-    tmp[g * 32 + c] = acc;
-    __syncthreads();
-    if ((int)threadIdx.x < 32 && col < ncols) {
-      float t = 0.f;
-      for (int gg = 0; gg < ng; ++gg) t += tmp[gg * 32 + c];
-      out[col] = t;
+// Column totals over all CTAs (partials of CTA b at p + b * stride; ncols a power of two >= 4), fixed order,
+// into smem out[0..ncols): neighbouring threads take neighbouring columns, the groups of threads every
+// G-th CTA with their loads in flight together, then a tree over the groups.  (One load at a time over
+// 608 CTAs' partials was the larger part of a step.)
+template <class T>
+__device__ __forceinline__ void grid_totals(const T* p, int nb, int64_t stride, int ncols, T* out, T* tmp) {
+  const int w = ncols < 32 ? ncols : 32, c = threadIdx.x % w, g = threadIdx.x / w, G = kBT / w;
+  for (int cb = 0; cb < ncols; cb += w) {
+    constexpr int B = 8;
+    T acc = T(0);
+    for (int b = g; b < nb; b += B * G) {
+      T v[B];
+#pragma unroll
+      for (int e = 0; e < B; ++e) v[e] = b + e * G < nb ? __ldcg(p + (int64_t)(b + e * G) * stride + cb + c) : T(0);
+#pragma unroll
+      for (int e = 0; e < B; ++e) acc += v[e];
     }
+    tmp[g * w + c] = acc;
     __syncthreads();
-  }
-}
-__device__ __forceinline__ void grid_totals_d(const double* pd, int nb, int64_t stride, int ncols, double* out,
-                                              double* tmp) {
-  const int c = threadIdx.x & 31, g = threadIdx.x >> 5, ng = kBT / 32;
-  for (int cb = 0; cb < ncols; cb += 32) {
-    const int col = cb + c;
-    double acc = 0.0;
-    if (col < ncols)
-      for (int b = g; b < nb; b += ng) acc += pd[(int64_t)b * stride + col];
-    tmp[g * 32 + c] = acc;
-    __syncthreads();
-    if ((int)threadIdx.x < 32 && col < ncols) {
-      double t = 0.0;
-      for (int gg = 0; gg < ng; ++gg) t += tmp[gg * 32 + c];
-      out[col] = t;
+    for (int h = G / 2; h >= 1; h >>= 1) {
+      if (g < h) tmp[g * w + c] += tmp[(g + h) * w + c];
+      __syncthreads();
     }
+    if (g == 0) out[cb + c] = tmp[c];
     __syncthreads();
   }
 }
 
-// Four CTAs per SM (64 registers, no spills): the SpMM phase is latency-bound on index -> p-row
-// gathers, and at two CTAs per SM (124 registers) only a quarter of the warp slots were occupied.
-__global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
-  __shared__ float4 red[kBT];
-  __shared__ double tmpd[kBT];
-  __shared__ float tmpf[kBT];
-  __shared__ float alpha[kBMaxK], beta[kBMaxK], gam[kBMaxK], gnew[kBMaxK], rn[kBMaxK], rmax[kBMaxK], pap[kBMaxK];
+// One CTA of 1024 threads per SM (64 registers): the SpMM phase is latency-bound on index -> p-row gathers
+// and wants full warp slots, the barriers and column totals want few CTAs.  256-thread CTAs, four per SM,
+// took 57 us a step for 64^3 unknowns x 16 columns; this form takes @@.
+__global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
+  extern __shared__ float4 red[];  // 2 * kBT
+  double* const tmpd = reinterpret_cast<double*>(red);  // kBT, between the reductions
+  float* const tmpf = reinterpret_cast<float*>(red + kBT);
+  __shared__ float alpha[kBMaxK], beta[kBMaxK], gam[kBMaxK], rmax[kBMaxK], pap[kBMaxK];
+  __shared__ float rg[2 * kBMaxK];  // |r|^2, then |r|; <r, z>
   __shared__ double bnorm[kBMaxK], relres[kBMaxK], tot64[2 * kBMaxK];
   __shared__ int frozen[kBMaxK], its[kBMaxK], status[kBMaxK];
-  __shared__ int s_flag;
 
   const int64_t n = a.n;
   const int kp = a.kp, q = a.q;
@@ -126,6 +125,8 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
   const int64_t r1 = r0 + rows < n ? r0 + rows : n;
   const int64_t nu = (r1 - r0) * q;   // (row, quad) units of this CTA
   const int cq = (int)threadIdx.x % q;
+  float* const rn = rg;
+  float* const gnew = rg + kp;
   float* pf = a.pf + (int64_t)blockIdx.x * 3 * kp;
   double* pd = a.pd + (int64_t)blockIdx.x * 2 * kp;
   const float4* P4 = reinterpret_cast<const float4*>(a.P);
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
       a.dinv[i] = dg != 0.f ? 1.f / dg : 1.f;
     }
   if (!grid_sync(a.gb)) return;
-  grid_totals_d(a.pd, nb, 2 * kp, kp, tot64, tmpd);
+  grid_totals<double>(a.pd, nb, 2 * kp, kp, tot64, tmpd);
   for (int c = threadIdx.x; c < kp; c += kBT) {
     const double bb = sqrt(tot64[c]);
     bnorm[c] = bb;
@@ -219,8 +220,8 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
     }
     __syncthreads();
     if (!grid_sync(a.gb)) return false;
-    grid_totals_d(a.pd + kp, nb, 2 * kp, kp, tot64, tmpd);
-    grid_totals_f(a.pf + 2 * kp, nb, 3 * kp, kp, gnew, tmpf);
+    grid_totals<double>(a.pd + kp, nb, 2 * kp, kp, tot64, tmpd);
+    grid_totals<float>(a.pf + 2 * kp, nb, 3 * kp, kp, gnew, tmpf);
     for (int c = threadIdx.x; c < kp; c += kBT) {
       if (frozen[c]) continue;
       const double rr = sqrt(tot64[c]);
@@ -253,15 +254,10 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
 
   int it = 0, nrep = 1;
   while (true) {
-    if (threadIdx.x == 0) {
-      int any = 0;
-      for (int c = 0; c < kp; ++c) any |= !frozen[c];
-      s_flag = any;
-    }
-    __syncthreads();
-    if (!s_flag) break;
+    if (!__syncthreads_or((int)threadIdx.x < kp && !frozen[threadIdx.x])) break;
     // ---- A: AP = A P, <p, Ap> ----
-    float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 parts[1] = {make_float4(0.f, 0.f, 0.f, 0.f)};
+    float4& part = parts[0];
     for (int64_t u = threadIdx.x; u < nu; u += kBT) {
       const int64_t i = r0 + u / q;
       const int32_t b = __ldg(a.indptr + i), e = __ldg(a.indptr + i + 1);
@@ -292,9 +288,10 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
       const float4 p = P4[i * q + cq];
       part.x += p.x * acc.x; part.y += p.y * acc.y; part.z += p.z * acc.z; part.w += p.w * acc.w;
     }
-    block_quad_partials(part, q, pf, red);
+    float* const to_a[1] = {pf};
+    block_quad_partials<1>(parts, q, to_a, red);
     if (!grid_sync(a.gb)) return;
-    grid_totals_f(a.pf, nb, 3 * kp, kp, pap, tmpf);
+    grid_totals<float>(a.pf, nb, 3 * kp, kp, pap, tmpf);
     for (int c = threadIdx.x; c < kp; c += kBT) {
       if (frozen[c]) { alpha[c] = 0.f; continue; }
       if (!(pap[c] > 0.f)) {
@@ -307,7 +304,8 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
     }
     __syncthreads();
     // ---- B: r -= alpha Ap, |r|^2, <r, z> (d += alpha p waits for phase C, which reads p anyway) ----
-    float4 prr = make_float4(0.f, 0.f, 0.f, 0.f), prz = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 sums[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    float4 &prr = sums[0], &prz = sums[1];
     const float4 al = make_float4(alpha[4 * cq], alpha[4 * cq + 1], alpha[4 * cq + 2], alpha[4 * cq + 3]);
     for (int64_t u = threadIdx.x; u < nu; u += kBT) {
       const int64_t i = r0 + u / q;
@@ -320,32 +318,27 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
       prr.x += r.x * r.x; prr.y += r.y * r.y; prr.z += r.z * r.z; prr.w += r.w * r.w;
       prz.x += r.x * di * r.x; prz.y += r.y * di * r.y; prz.z += r.z * di * r.z; prz.w += r.w * di * r.w;
     }
-    block_quad_partials(prr, q, pf + kp, red);
-    block_quad_partials(prz, q, pf + 2 * kp, red);
+    float* const to_b[2] = {pf + kp, pf + 2 * kp};
+    block_quad_partials<2>(sums, q, to_b, red);
     if (!grid_sync(a.gb)) return;
-    grid_totals_f(a.pf + kp, nb, 3 * kp, kp, rn, tmpf);
-    grid_totals_f(a.pf + 2 * kp, nb, 3 * kp, kp, gnew, tmpf);
+    grid_totals<float>(a.pf + kp, nb, 3 * kp, 2 * kp, rg, tmpf);  // rn and gnew
     ++it;
-    if (threadIdx.x == 0) {
-      int trig = 0;
-      for (int c = 0; c < kp; ++c) {
-        if (frozen[c]) continue;
-        its[c] = it;
-        const float r = sqrtf(rn[c]);
-        rn[c] = r;
-        if (!(r == r)) {
-          status[c] = COLAGB_SYS_NAN;
-          frozen[c] = 1;
-          continue;
-        }
-        if (r <= (float)a.inner_tol * rmax[c] || r <= (float)a.tol) trig = 1;
+    int trig = it >= a.max_inner;
+    if ((int)threadIdx.x < kp && !frozen[threadIdx.x]) {
+      const int c = threadIdx.x;
+      its[c] = it;
+      const float r = sqrtf(rn[c]);
+      rn[c] = r;
+      if (!(r == r)) {
+        status[c] = COLAGB_SYS_NAN;
+        frozen[c] = 1;
+      } else if (r <= (float)a.inner_tol * rmax[c] || r <= (float)a.tol) {
+        trig = 1;
       }
-      if (it >= a.max_inner) trig = 1;
-      s_flag = trig;
     }
-    __syncthreads();
-    const bool dpend = !s_flag;  // a replacement has already added this step's alpha p to x
-    if (s_flag) {
+    trig = __syncthreads_or(trig);
+    const bool dpend = !trig;  // a replacement has already added this step's alpha p to x
+    if (trig) {
       if (!replace(false)) return;
       ++nrep;
       if (it >= a.max_inner || nrep > a.max_sweeps) break;
@@ -389,6 +382,8 @@ __global__ void __launch_bounds__(kBT, 4) k_block_ir(const BlockArgs a) {
   }
 }
 
+constexpr size_t kBlockSmem = 2 * kBT * sizeof(float4);
+
 int block_padded_width(int64_t k) {
   int kp = 4;
   while (kp < k) kp *= 2;
@@ -412,11 +407,11 @@ size_t block_workspace_bytes(int64_t n, int64_t S, int nb_max) {
 
 int block_grid_blocks() {
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_ir, kBT, 0) != cudaSuccess || occ < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_ir, kBT, kBlockSmem) != cudaSuccess || occ < 1) {
     cudaGetLastError();
     return 0;
   }
-  return num_sms() * (occ < 4 ? occ : 4);
+  return num_sms();
 }
 
 // One shared-matrix block of up to kBMaxK right-hand sides (B, X: (S, n) FP64).
@@ -462,14 +457,13 @@ int block_pcg_solve(const colagb_batched_csr* A, const double* B, double* X, con
     a.inner_tol = prm->inner_tol;
     a.max_inner = prm->max_inner_iters;
     a.max_sweeps = prm->max_sweeps;
-    a.gb.count = bar;
-    a.gb.generation = bar + 1;
+    a.gb.arrivals = reinterpret_cast<unsigned long long*>(bar);
     a.gb.err = reinterpret_cast<int*>(bar + 2);
     a.gb.nblocks = (unsigned)nb;
     a.gb.spin_limit = prm->spin_limit > 0 ? prm->spin_limit : kDefaultSpinLimit;
     COLAGB_CUDA(cudaMemsetAsync(bar, 0, 8 * sizeof(unsigned int), st));
     void* args[] = {&a};
-    COLAGB_CUDA(cudaLaunchCooperativeKernel((const void*)k_block_ir, dim3(nb), dim3(kBT), args, 0, st));
+    COLAGB_CUDA(cudaLaunchCooperativeKernel((const void*)k_block_ir, dim3(nb), dim3(kBT), args, kBlockSmem, st));
     int h[2] = {0, 0};
     COLAGB_CUDA(cudaMemcpyAsync(&h[0], bar + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
     COLAGB_CUDA(cudaMemcpyAsync(&h[1], nrep, sizeof(int), cudaMemcpyDeviceToHost, st));

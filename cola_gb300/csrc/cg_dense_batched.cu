@@ -491,8 +491,7 @@ extern "C" int colagb_cg_dense_batched_solve(int64_t num_systems, const int32_t*
   a.out_status = per_system_status;
   a.tol = tol;
   a.max_iters = max_iters;
-  a.gb.count = bar;
-  a.gb.generation = bar + 1;
+  a.gb.arrivals = reinterpret_cast<unsigned long long*>(bar);
   a.gb.err = reinterpret_cast<int*>(bar + 2);
   a.gb.spin_limit = kDefaultSpinLimit;
   cudaStream_t st = as_stream(stream);

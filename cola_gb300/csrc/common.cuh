@@ -103,20 +103,18 @@ __device__ __forceinline__ T block_sum(T v, T* scratch) {
 
 // ---- bounded grid barrier ---------------------------------------------------------------
 // Used only by kernels launched with cudaLaunchCooperativeKernel (all CTAs co-resident).
-// Sense/generation barrier on two global words.  A CTA that spins more than `spin_limit`
-// times records COLAGB_ERR_TIMEOUT in *err and reports failure; every caller then leaves the
-// kernel, so a lost CTA can never hang the GPU.
+// One 64-bit arrival counter in global memory, zero at launch, that only grows: barrier number g is through
+// when g * nblocks CTAs have arrived.  An arrival is one atomic and the wait polls with acquire loads
+// (1.3 us on 152 CTAs, 1.5 us on 304; the earlier count / generation pair took a second atomic and
+// naps).  A CTA that polls more than `spin_limit` times records COLAGB_ERR_TIMEOUT in *err and reports
+// failure; every caller then leaves the kernel, so a lost CTA can never hang the GPU.
 struct GridBarrier {
-  unsigned int* count;
-  unsigned int* generation;
+  unsigned long long* arrivals;
   int* err;
   unsigned int nblocks;
   long long spin_limit;
 };
 
-__device__ __forceinline__ unsigned int ld_volatile(const unsigned int* p) {
-  return *reinterpret_cast<const volatile unsigned int*>(p);
-}
 __device__ __forceinline__ int ld_volatile_i(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
 // Returns true when every CTA arrived; false on timeout or when another CTA flagged an error.
@@ -125,26 +123,21 @@ __device__ __forceinline__ bool grid_sync(const GridBarrier& gb) {
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
-    const unsigned int gen = ld_volatile(gb.generation);
     __threadfence();
-    const unsigned int arrived = atomicAdd(gb.count, 1u);
-    if (arrived == gb.nblocks - 1) {
-      atomicExch(gb.count, 0u);
-      __threadfence();
-      atomicAdd(gb.generation, 1u);
-    } else {
-      long long spins = 0;
-      while (ld_volatile(gb.generation) == gen) {
-        if (ld_volatile_i(gb.err) != 0) { ok = 0; break; }
-        if (++spins > gb.spin_limit) {
-          atomicCAS(gb.err, 0, COLAGB_ERR_TIMEOUT);
-          ok = 0;
-          break;
-        }
-        __nanosleep(20);
+    const unsigned long long before = atomicAdd(gb.arrivals, 1ull);
+    const unsigned long long target = (before / gb.nblocks + 1) * gb.nblocks;
+    long long spins = 0;
+    while (true) {
+      unsigned long long v;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(gb.arrivals) : "memory");
+      if (v >= target) break;
+      if (ld_volatile_i(gb.err) != 0) { ok = 0; break; }
+      if (++spins > gb.spin_limit) {
+        atomicCAS(gb.err, 0, COLAGB_ERR_TIMEOUT);
+        ok = 0;
+        break;
       }
     }
-    __threadfence();
     if (ld_volatile_i(gb.err) != 0) ok = 0;
     s_ok = ok;
   }
@@ -158,6 +151,6 @@ __device__ __forceinline__ bool grid_sync(const GridBarrier& gb) {
 // forced after this many steps without one.  Converging FSAI-PCG replaces far more often.
 constexpr int kJudgeSteps = 1000;
 
-constexpr long long kDefaultSpinLimit = 20000000LL;  // ~ a few seconds of 20 ns naps
+constexpr long long kDefaultSpinLimit = 20000000LL;  // polls of about half a microsecond: ten seconds
 
 }  // namespace colagb

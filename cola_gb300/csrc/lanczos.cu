@@ -115,10 +115,10 @@ __device__ __forceinline__ void lz_partials4(int64_t n, int64_t bs, const float*
 #pragma unroll
     for (int u = 0; u < 3; ++u)
       if (r + u * stride < n) {
-        acc[0].x += x[u].x * y[u].x;
-        acc[0].y += x[u].y * y[u].y;
-        acc[0].z += x[u].z * y[u].z;
-        acc[0].w += x[u].w * y[u].w;
+        acc[0].x = fmaf(x[u].x, y[u].x, acc[0].x);
+        acc[0].y = fmaf(x[u].y, y[u].y, acc[0].y);
+        acc[0].z = fmaf(x[u].z, y[u].z, acc[0].z);
+        acc[0].w = fmaf(x[u].w, y[u].w, acc[0].w);
       }
   }
   float4 tot;
@@ -308,10 +308,11 @@ struct LzStep {
 };
 
 __device__ __forceinline__ float lz_term(float w, float d, float vi, float sb, float vim1) {
-  w -= d * vi + sb * vim1;
-  return w;
+  return w - fmaf(d, vi, sb * vim1);
 }
 
+// (fmaf is written out where an addition is predicated: the compiler may otherwise select the product and
+// add it, rounding twice.)
 // sum over j = 1..i, in that order, of V[j] h[j] at one / two / four entries (offset o, column(s) of h).  The
 // loads of a batch of slots are issued together, the last batch predicated: a remainder loop would wait
 // for one load at a time (74 us instead of 30 for 20 slots of 1.8M entries).
@@ -329,7 +330,7 @@ __device__ __forceinline__ float lz_comb1(const float* basis, int64_t N, int64_t
       }
 #pragma unroll
     for (int q = 0; q < B; ++q)
-      if (j + q <= i) acc += x[q] * c[q];
+      if (j + q <= i) acc = fmaf(x[q], c[q], acc);
   }
   return acc;
 }
@@ -339,24 +340,21 @@ __device__ __forceinline__ float2 lz_comb2(const float* basis, int64_t N, int64_
   const float* v = basis + N + o;
   for (int j = 1; j <= i; j += B, v += B * N) {
     float2 x[B];
-    float c[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (j + q <= i) x[q] = __ldg(reinterpret_cast<const float2*>(v + q * N));
 #pragma unroll
     for (int q = 0; q < B; ++q)
       if (j + q <= i) {
-        x[q] = __ldg(reinterpret_cast<const float2*>(v + q * N));
-        c[q] = __ldg(h + j + q);
-      }
-#pragma unroll
-    for (int q = 0; q < B; ++q)
-      if (j + q <= i) {
-        acc.x += x[q].x * c[q];
-        acc.y += x[q].y * c[q];
+        const float c = h[j + q];
+        acc.x = fmaf(x[q].x, c, acc.x);
+        acc.y = fmaf(x[q].y, c, acc.y);
       }
   }
   return acc;
 }
+template <bool ONE, int B>
 __device__ __forceinline__ float4 lz_comb4(const float* basis, int64_t N, int64_t o, const float* h, int64_t bs, int i) {
-  constexpr int B = 8;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* v = basis + N + o;
   for (int j = 1; j <= i; j += B, v += B * N) {
@@ -364,25 +362,25 @@ __device__ __forceinline__ float4 lz_comb4(const float* basis, int64_t N, int64_
 #pragma unroll
     for (int q = 0; q < B; ++q)
       if (j + q <= i) x[q] = __ldg(reinterpret_cast<const float4*>(v + q * N));
-    if (bs == 1) {
+    if constexpr (ONE) {
 #pragma unroll
       for (int q = 0; q < B; ++q)
         if (j + q <= i) {
           const float c = __ldg(h + j + q);
-          acc.x += x[q].x * c;
-          acc.y += x[q].y * c;
-          acc.z += x[q].z * c;
-          acc.w += x[q].w * c;
+          acc.x = fmaf(x[q].x, c, acc.x);
+          acc.y = fmaf(x[q].y, c, acc.y);
+          acc.z = fmaf(x[q].z, c, acc.z);
+          acc.w = fmaf(x[q].w, c, acc.w);
         }
     } else {
 #pragma unroll
       for (int q = 0; q < B; ++q)
         if (j + q <= i) {
           const float4 c = __ldg(reinterpret_cast<const float4*>(h + (int64_t)(j + q) * bs));
-          acc.x += x[q].x * c.x;
-          acc.y += x[q].y * c.y;
-          acc.z += x[q].z * c.z;
-          acc.w += x[q].w * c.w;
+          acc.x = fmaf(x[q].x, c.x, acc.x);
+          acc.y = fmaf(x[q].y, c.y, acc.y);
+          acc.z = fmaf(x[q].z, c.z, acc.z);
+          acc.w = fmaf(x[q].w, c.w, acc.w);
         }
     }
   }
@@ -403,6 +401,11 @@ __global__ void __launch_bounds__(512, 2) k_lz_proj1(const __grid_constant__ LzS
   const int n2 = (int)((r1 - r0) / 2), n4 = n2 / 2;
   float2* w2 = reinterpret_cast<float2*>(a.w + r0);
   const float d = MODE == LZ_TERMS_PROJ ? a.diag[i - 1] : 0.f, sb = MODE == LZ_TERMS_PROJ ? a.subdiag[i - 1] : 0.f;
+  float* const hs = reinterpret_cast<float*>(wsm) + a.chunk;  // the coefficients, behind the run
+  if (MODE == LZ_SUB_PROJ) {
+    for (int j = threadIdx.x; j <= i; j += blockDim.x) hs[j] = s.hbuf[j];
+    __syncthreads();
+  }
   for (int u = threadIdx.x; u < n2; u += blockDim.x) {
     float2 x = w2[u];
     if (MODE == LZ_TERMS_PROJ) {
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(512, 2) k_lz_proj1(const __grid_constant__ LzS
       x.x = lz_term(x.x, d, p.x, sb, q.x);
       x.y = lz_term(x.y, d, p.y, sb, q.y);
     } else {
-      const float2 c = lz_comb2(a.basis, n, r0 + 2 * u, s.hbuf, i);
+      const float2 c = lz_comb2(a.basis, n, r0 + 2 * u, hs, i);
       x.x -= c.x;
       x.y -= c.y;
     }
@@ -432,8 +435,9 @@ __global__ void __launch_bounds__(512, 2) k_lz_proj1(const __grid_constant__ LzS
       for (int q = 0; q < B; ++q)
         if (u + 32 * q < n4) {
           const float4 p = v[q], x = wsm[u + 32 * q];
-          if (q % 2 == 0) acc0 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
-          else acc1 += p.x * x.x + p.y * x.y + p.z * x.z + p.w * x.w;
+          const float d4 = fmaf(p.w, x.w, fmaf(p.z, x.z, fmaf(p.x, x.x, p.y * x.y)));
+          if (q % 2 == 0) acc0 += d4;
+          else acc1 += d4;
         }
     }
     const float t = warp_sum(acc0 + acc1);
@@ -467,7 +471,7 @@ __global__ void __launch_bounds__(512, 2) k_lz_projq(const __grid_constant__ LzS
       x.z = lz_term(x.z, __ldg(dg + 2 * m), p.z, __ldg(sb + 2 * (m + 1)), q.z);
       x.w = lz_term(x.w, __ldg(dg + 3 * m), p.w, __ldg(sb + 3 * (m + 1)), q.w);
     } else {
-      const float4 c = lz_comb4(a.basis, N, r0 * bs + 4 * u, s.hbuf + b, bs, i);
+      const float4 c = lz_comb4<false, 8>(a.basis, N, r0 * bs + 4 * u, s.hbuf + b, bs, i);
       x.x -= c.x;
       x.y -= c.y;
       x.z -= c.z;
@@ -492,7 +496,7 @@ __global__ void __launch_bounds__(512, 2) k_lz_projq(const __grid_constant__ LzS
         if (u + 32 * q < n4) {
           const float4 p = v[q], x = wsm[u + 32 * q];
           float4& d = q % 2 == 0 ? acc : acc2;
-          d.x += p.x * x.x; d.y += p.y * x.y; d.z += p.z * x.z; d.w += p.w * x.w;
+          d.x = fmaf(p.x, x.x, d.x); d.y = fmaf(p.y, x.y, d.y); d.z = fmaf(p.z, x.z, d.z); d.w = fmaf(p.w, x.w, d.w);
         }
     }
     acc.x += acc2.x; acc.y += acc2.y; acc.z += acc2.z; acc.w += acc2.w;
@@ -602,7 +606,9 @@ __global__ void __launch_bounds__(1024) k_lz_reduce32(int nblk, int64_t bs, int6
 
 // The last subtraction with the sums of squares of lz_colsum on the way (the same rows per thread), then
 // subdiag[b][i] = |w|, i += 1 and the stop test of lanczos_fact.cond_fun in the last CTA.
-__global__ void __launch_bounds__(256, 4) k_lz_fin(const __grid_constant__ LzStep a, float* subdiag, double tol) {
+// FORM 0: any bs; 1: float4 of blocks with bs % 4 == 0; 2: float4 of one column.
+template <int FORM>
+__global__ void __launch_bounds__(256, FORM == 1 ? 4 : 2) k_lz_fin(const __grid_constant__ LzStep a, float* subdiag, double tol) {
   const LzState<float>& s = a.s;
   if (*s.done) return;
   __shared__ float4 smem4[256];
@@ -610,37 +616,42 @@ __global__ void __launch_bounds__(256, 4) k_lz_fin(const __grid_constant__ LzSte
   const int i = *s.step, t = threadIdx.x;
   const int64_t n = a.n, bs = a.bs, N = n * bs;
   float* const out = s.npart + (int64_t)blockIdx.x * bs;
-  const bool al = (reinterpret_cast<uintptr_t>(a.basis) % 16) == 0 && (reinterpret_cast<uintptr_t>(a.w) % 16) == 0;
-  const bool one = bs == 1 && n % 4 == 0;
-  if (al && (one || (bs % 4 == 0 && bs <= 1024))) {
+  constexpr bool one = FORM == 2;
+  if constexpr (FORM != 0) {
     const int64_t rows = one ? n / 4 : n;  // a single column: rows of four entries
     const int qd = one ? 1 : (int)(bs / 4), rpp = 256 / qd;
     const int my_q = t % qd, my_r = t / qd;
     float4 acc[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto term = [&](int64_t r, float4& d) {
-      const int64_t o = (r * qd + my_q) * 4;
-      float4 x = *reinterpret_cast<const float4*>(a.w + o);
-      const float4 c = lz_comb4(a.basis, N, o, s.hbuf + (one ? 0 : 4 * my_q), bs, i);
-      x.x -= c.x;
-      x.y -= c.y;
-      x.z -= c.z;
-      x.w -= c.w;
-      *reinterpret_cast<float4*>(a.w + o) = x;
-      d.x += x.x * x.x;
-      d.y += x.y * x.y;
-      d.z += x.z * x.z;
-      d.w += x.w * x.w;
-    };
     if (my_r < rpp) {
+      // rounds of four rows on four accumulators, the last one to three rows all on the first
       const int64_t stride = (int64_t)rpp * gridDim.x;
-      int64_t r = (int64_t)blockIdx.x * rpp + my_r;
-      for (; r + 3 * stride < rows; r += 4 * stride) {
+      for (int64_t r = (int64_t)blockIdx.x * rpp + my_r; r < rows; r += 4 * stride) {
+        const bool full = r + 3 * stride < rows;
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+          const int64_t ru = r + u * stride;
+          if (ru >= rows) break;
+          const int64_t o = (ru * qd + my_q) * 4;
+          float4 x = *reinterpret_cast<const float4*>(a.w + o);
+          const float4 c = lz_comb4<one, one ? 16 : 6>(a.basis, N, o, s.hbuf + (one ? 0 : 4 * my_q), bs, i);
+          x.x -= c.x;
+          x.y -= c.y;
+          x.z -= c.z;
+          x.w -= c.w;
+          *reinterpret_cast<float4*>(a.w + o) = x;
+          const int to = full ? u : 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) term(r + u * stride, acc[u]);
+          for (int d = 0; d < 4; ++d)
+            if (to == d) {
+              acc[d].x = fmaf(x.x, x.x, acc[d].x);
+              acc[d].y = fmaf(x.y, x.y, acc[d].y);
+              acc[d].z = fmaf(x.z, x.z, acc[d].z);
+              acc[d].w = fmaf(x.w, x.w, acc[d].w);
+            }
+        }
       }
-      for (; r < rows; r += stride) term(r, acc[0]);
     }
     float4 tot;
     tot.x = (acc[0].x + acc[1].x) + (acc[2].x + acc[3].x);
@@ -707,7 +718,7 @@ struct LzForm {
   int64_t chunk = 0;
   size_t smem = 0;
 };
-static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, LzForm& f) {
+static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, int64_t slots, LzForm& f) {
   const bool al = (uintptr_t)basis % 16 == 0;
   f.blocks = nb;
   f.chunk = ceil_div(n, (int64_t)nb);
@@ -716,8 +727,12 @@ static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, LzForm& f)
   else if (bs >= 4 && bs <= 128 && (bs & (bs - 1)) == 0 && al) step = 128 / bs;
   if (step == 0) return COLAGB_OK;
   const int64_t chunk = ceil_div(f.chunk, step) * step;  // a whole number of 128-float warp steps
-  const size_t smem = (size_t)(chunk * bs) * sizeof(float);
+  size_t smem = (size_t)(chunk * bs) * sizeof(float);
   if (smem > 160 * 1024) return COLAGB_OK;
+  if (bs == 1) {  // the single-vector form keeps the coefficients in shared memory, too
+    smem += (size_t)slots * sizeof(float);
+    if (smem > 220 * 1024) return COLAGB_OK;
+  }
   f.form = bs == 1 ? 0 : 1;
   f.chunk = chunk;
   f.blocks = (int)ceil_div(n, chunk);
@@ -750,7 +765,12 @@ static int lz_step_f32(const LzForm& f, const LzStep& a, int i, int nb, float* d
   k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
   lz_project<LZ_SUB_PROJ>(f, a, i, st);
   k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
-  k_lz_fin<<<nb, 256, 0, st>>>(a, subdiag, tol);
+  // the 128-bit form where lz_colsum takes it: blocks of 4, 8, ... columns and single ones with n % 4 == 0
+  const bool quads = (uintptr_t)a.basis % 16 == 0 && (uintptr_t)a.w % 16 == 0 &&
+                     ((a.bs == 1 && a.n % 4 == 0) || (a.bs % 4 == 0 && a.bs <= 1024));
+  if (!quads) k_lz_fin<0><<<nb, 256, 0, st>>>(a, subdiag, tol);
+  else if (a.bs == 1) k_lz_fin<2><<<nb, 256, 0, st>>>(a, subdiag, tol);
+  else k_lz_fin<1><<<nb, 256, 0, st>>>(a, subdiag, tol);
   return COLAGB_OK;
 }
 
@@ -1420,7 +1440,7 @@ static int lanczos_t(const colagb_op* A, const T* V0, int64_t ldv0, int64_t bs, 
   const size_t blk = (size_t)n * bs;
   const GsPlan plan = gs_plan<T>(basis, n, bs, nb);
   LzForm form;
-  if constexpr (std::is_same<T, float>::value) COLAGB_TRY(lz_form(basis, n, bs, nb, form));
+  if constexpr (std::is_same<T, float>::value) COLAGB_TRY(lz_form(basis, n, bs, nb, (int64_t)m + 2, form));
   auto scale = [&](T* v) {
     if constexpr (std::is_same<T, float>::value)
       if (plan.vec == 4) {
