@@ -43,6 +43,7 @@ struct BlockArgs {
   int32_t* out_nrep;            // (1,) replacement count
   double tol, inner_tol;
   int max_inner, max_sweeps, jacobi;
+  int r_resident;               // r of the CTA's rows is kept in shared memory
   GridBarrier gb;
 };
 
@@ -106,8 +107,12 @@ __device__ __forceinline__ void grid_totals(const T* p, int nb, int64_t stride, 
 }
 
 // One CTA of 1024 threads per SM (64 registers): the SpMM phase is latency-bound on index -> p-row gathers
-// and wants full warp slots, the barriers and column totals want few CTAs.  256-thread CTAs, four per SM,
-// took 57 us a step for 64^3 unknowns x 16 columns; this form takes @@.
+// and wants full warp slots, the barriers and column totals want few CTAs; r of the CTA's rows stays in
+// shared memory where it takes at most half of it (the rest caches the gathers of p).  us a step for 64^3
+// unknowns x 16 columns, FP32: 57 with 256-thread CTAs, four per SM, and totals read one partial after
+// another; 43 in this shape; 41 with two units of the vector phases in flight; 40 with eight entries' indices
+// ahead of their gathers; 37 with r resident.  Rows of the matrix resident as well took the L1 from the
+// gathers (60).
 __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
   extern __shared__ float4 red[];  // 2 * kBT
   double* const tmpd = reinterpret_cast<double*>(red);  // kBT, between the reductions
@@ -123,14 +128,17 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
   const int64_t rows = ceil_div(n, nb);
   const int64_t r0 = (int64_t)blockIdx.x * rows < n ? (int64_t)blockIdx.x * rows : n;
   const int64_t r1 = r0 + rows < n ? r0 + rows : n;
-  const int64_t nu = (r1 - r0) * q;   // (row, quad) units of this CTA
+  const int nu = (int)((r1 - r0) * q);   // (row, quad) units of this CTA
+  int qs = 0;                            // log2 q
+  while ((1 << qs) < q) ++qs;
   const int cq = (int)threadIdx.x % q;
   float* const rn = rg;
   float* const gnew = rg + kp;
   float* pf = a.pf + (int64_t)blockIdx.x * 3 * kp;
   double* pd = a.pd + (int64_t)blockIdx.x * 2 * kp;
   const float4* P4 = reinterpret_cast<const float4*>(a.P);
-  float4* R4 = reinterpret_cast<float4*>(a.R);
+  float4* const R4 = a.r_resident ? red + 2 * kBT : reinterpret_cast<float4*>(a.R) + r0 * q;  // the CTA's units
+  float* const Rf = reinterpret_cast<float*>(R4);
   float4* Pw4 = reinterpret_cast<float4*>(a.P);
   float4* AP4 = reinterpret_cast<float4*>(a.AP);
   float4* D4 = reinterpret_cast<float4*>(a.D);
@@ -200,7 +208,7 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
           ax += (double)a.vals[j] * a.X64[(int64_t)a.indices[j] * kp + col];
       const double rv = frozen[col] ? 0.0 : a.Bn[i * kp + col] - ax;
       const float rf = (float)rv;
-      a.R[i * kp + col] = rf;
+      Rf[u] = rf;
       acc_rr += rv * rv;
       acc_rz += rf * (a.jacobi ? a.dinv[i] : 1.f) * rf;
     }
@@ -244,9 +252,9 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
   for (int c = threadIdx.x; c < kp; c += kBT) gam[c] = gnew[c];
   __syncthreads();
   // p = z
-  for (int64_t u = threadIdx.x; u < nu; u += kBT) {
-    const int64_t i = r0 + u / q;
-    const float4 r = R4[i * q + cq];
+  for (int u = threadIdx.x; u < nu; u += kBT) {
+    const int64_t i = r0 + (u >> qs);
+    const float4 r = R4[u];
     const float d = a.jacobi ? a.dinv[i] : 1.f;
     Pw4[i * q + cq] = make_float4(d * r.x, d * r.y, d * r.z, d * r.w);
   }
@@ -258,29 +266,32 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
     // ---- A: AP = A P, <p, Ap> ----
     float4 parts[1] = {make_float4(0.f, 0.f, 0.f, 0.f)};
     float4& part = parts[0];
-    for (int64_t u = threadIdx.x; u < nu; u += kBT) {
-      const int64_t i = r0 + u / q;
+    for (int u = threadIdx.x; u < nu; u += kBT) {
+      const int64_t i = r0 + (u >> qs);
       const int32_t b = __ldg(a.indptr + i), e = __ldg(a.indptr + i + 1);
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      // entries in groups of four: the group's indices and values, then its four p-row gathers, are
-      // in flight together (one dependent index -> gather round trip per entry made this phase
-      // latency-bound); the products are added in entry order as before
-      for (int32_t j0 = b; j0 < e; j0 += 4) {
-        int32_t col[4];
-        float v[4];
+      // eight entries' indices and values at a time, then their p-row gathers four by four, so that the
+      // loads of a group are in flight together; the products are added in entry order
+      for (int32_t j0 = b; j0 < e; j0 += 8) {
+        int32_t col[8];
+        float v[8];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
+        for (int t = 0; t < 8; ++t) {
           const bool ok = j0 + t < e;
           col[t] = ok ? __ldg(a.indices + j0 + t) : 0;
           v[t] = ok ? __ldg(a.vals + j0 + t) : 0.f;
         }
-        float4 x[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) x[t] = j0 + t < e ? P4[(int64_t)col[t] * q + cq] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int h = 0; h < 8; h += 4) {
+          float4 x[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          if (j0 + t < e) {
-            acc.x += v[t] * x[t].x; acc.y += v[t] * x[t].y; acc.z += v[t] * x[t].z; acc.w += v[t] * x[t].w;
+          for (int t = 0; t < 4; ++t)
+            x[t] = j0 + h + t < e ? P4[(int64_t)col[h + t] * q + cq] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            if (j0 + h + t < e) {
+              acc.x += v[h + t] * x[t].x; acc.y += v[h + t] * x[t].y; acc.z += v[h + t] * x[t].z; acc.w += v[h + t] * x[t].w;
+            }
           }
         }
       }
@@ -307,16 +318,22 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
     float4 sums[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     float4 &prr = sums[0], &prz = sums[1];
     const float4 al = make_float4(alpha[4 * cq], alpha[4 * cq + 1], alpha[4 * cq + 2], alpha[4 * cq + 3]);
-    for (int64_t u = threadIdx.x; u < nu; u += kBT) {
-      const int64_t i = r0 + u / q;
-      const int64_t e = i * q + cq;
-      const float4 ap = AP4[e];
-      float4 r = R4[e];
-      r.x -= al.x * ap.x; r.y -= al.y * ap.y; r.z -= al.z * ap.z; r.w -= al.w * ap.w;
-      R4[e] = r;
-      const float di = a.jacobi ? a.dinv[i] : 1.f;
-      prr.x += r.x * r.x; prr.y += r.y * r.y; prr.z += r.z * r.z; prr.w += r.w * r.w;
-      prz.x += r.x * di * r.x; prz.y += r.y * di * r.y; prz.z += r.z * di * r.z; prz.w += r.w * di * r.w;
+    // unit u is element r0 * q + u: two units in flight, the second one's terms zero past the end
+    for (int u = threadIdx.x; u < nu; u += 2 * kBT) {
+      const int64_t e0 = r0 * q + u, e1 = u + kBT < nu ? e0 + kBT : e0;
+      const float4 ap0 = AP4[e0], ap1 = AP4[e1];
+      float4 x0 = R4[u], x1 = R4[u + (int)(e1 - e0)];
+      const float d0 = a.jacobi ? a.dinv[e0 >> qs] : 1.f, d1 = a.jacobi ? a.dinv[e1 >> qs] : 1.f;
+      x0.x -= al.x * ap0.x; x0.y -= al.y * ap0.y; x0.z -= al.z * ap0.z; x0.w -= al.w * ap0.w;
+      R4[u] = x0;
+      prr.x += x0.x * x0.x; prr.y += x0.y * x0.y; prr.z += x0.z * x0.z; prr.w += x0.w * x0.w;
+      prz.x += x0.x * d0 * x0.x; prz.y += x0.y * d0 * x0.y; prz.z += x0.z * d0 * x0.z; prz.w += x0.w * d0 * x0.w;
+      if (e1 != e0) {
+        x1.x -= al.x * ap1.x; x1.y -= al.y * ap1.y; x1.z -= al.z * ap1.z; x1.w -= al.w * ap1.w;
+        R4[u + kBT] = x1;
+        prr.x += x1.x * x1.x; prr.y += x1.y * x1.y; prr.z += x1.z * x1.z; prr.w += x1.w * x1.w;
+        prz.x += x1.x * d1 * x1.x; prz.y += x1.y * d1 * x1.y; prz.z += x1.z * d1 * x1.z; prz.w += x1.w * d1 * x1.w;
+      }
     }
     float* const to_b[2] = {pf + kp, pf + 2 * kp};
     block_quad_partials<2>(sums, q, to_b, red);
@@ -350,18 +367,20 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
     }
     __syncthreads();
     const float4 be = make_float4(beta[4 * cq], beta[4 * cq + 1], beta[4 * cq + 2], beta[4 * cq + 3]);
-    for (int64_t u = threadIdx.x; u < nu; u += kBT) {
-      const int64_t i = r0 + u / q;
-      const int64_t e = i * q + cq;
-      const float4 r = R4[e], p = P4[e];
+    for (int u = threadIdx.x; u < nu; u += 2 * kBT) {
+      const int64_t e0 = r0 * q + u, e1 = u + kBT < nu ? e0 + kBT : e0;
+      const float4 x0 = R4[u], x1 = R4[u + (int)(e1 - e0)], p0 = P4[e0], p1 = P4[e1];
+      const float d0 = a.jacobi ? a.dinv[e0 >> qs] : 1.f, d1 = a.jacobi ? a.dinv[e1 >> qs] : 1.f;
       if (dpend) {
-        float4 d = D4[e];
-        d.x += al.x * p.x; d.y += al.y * p.y; d.z += al.z * p.z; d.w += al.w * p.w;
-        D4[e] = d;
+        float4 y0 = D4[e0], y1 = D4[e1];
+        y0.x += al.x * p0.x; y0.y += al.y * p0.y; y0.z += al.z * p0.z; y0.w += al.w * p0.w;
+        D4[e0] = y0;
+        y1.x += al.x * p1.x; y1.y += al.y * p1.y; y1.z += al.z * p1.z; y1.w += al.w * p1.w;
+        if (e1 != e0) D4[e1] = y1;
       }
-      const float di = a.jacobi ? a.dinv[i] : 1.f;
-      Pw4[e] = make_float4(di * r.x + be.x * p.x, di * r.y + be.y * p.y, di * r.z + be.z * p.z,
-                           di * r.w + be.w * p.w);
+      Pw4[e0] = make_float4(d0 * x0.x + be.x * p0.x, d0 * x0.y + be.y * p0.y, d0 * x0.z + be.z * p0.z, d0 * x0.w + be.w * p0.w);
+      if (e1 != e0)
+        Pw4[e1] = make_float4(d1 * x1.x + be.x * p1.x, d1 * x1.y + be.y * p1.y, d1 * x1.z + be.z * p1.z, d1 * x1.w + be.w * p1.w);
     }
     if (!grid_sync(a.gb)) return;
   }
@@ -382,7 +401,7 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
   }
 }
 
-constexpr size_t kBlockSmem = 2 * kBT * sizeof(float4);
+constexpr size_t kBlockRed = 2 * kBT * sizeof(float4);
 
 int block_padded_width(int64_t k) {
   int kp = 4;
@@ -407,7 +426,7 @@ size_t block_workspace_bytes(int64_t n, int64_t S, int nb_max) {
 
 int block_grid_blocks() {
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_ir, kBT, kBlockSmem) != cudaSuccess || occ < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_block_ir, kBT, kBlockRed) != cudaSuccess || occ < 1) {
     cudaGetLastError();
     return 0;
   }
@@ -457,13 +476,18 @@ int block_pcg_solve(const colagb_batched_csr* A, const double* B, double* X, con
     a.inner_tol = prm->inner_tol;
     a.max_inner = prm->max_inner_iters;
     a.max_sweeps = prm->max_sweeps;
+    // r in shared memory where the rows' share is at most half of it: three of a step's vector streams less
+    const size_t r_bytes = (size_t)ceil_div(n, (int64_t)nb) * kp * sizeof(float);
+    a.r_resident = r_bytes <= 120 * 1024;
+    const size_t smem = kBlockRed + (a.r_resident ? r_bytes : 0);
+    COLAGB_CUDA(cudaFuncSetAttribute(k_block_ir, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     a.gb.arrivals = reinterpret_cast<unsigned long long*>(bar);
     a.gb.err = reinterpret_cast<int*>(bar + 2);
     a.gb.nblocks = (unsigned)nb;
     a.gb.spin_limit = prm->spin_limit > 0 ? prm->spin_limit : kDefaultSpinLimit;
     COLAGB_CUDA(cudaMemsetAsync(bar, 0, 8 * sizeof(unsigned int), st));
     void* args[] = {&a};
-    COLAGB_CUDA(cudaLaunchCooperativeKernel((const void*)k_block_ir, dim3(nb), dim3(kBT), args, kBlockSmem, st));
+    COLAGB_CUDA(cudaLaunchCooperativeKernel((const void*)k_block_ir, dim3(nb), dim3(kBT), args, smem, st));
     int h[2] = {0, 0};
     COLAGB_CUDA(cudaMemcpyAsync(&h[0], bar + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
     COLAGB_CUDA(cudaMemcpyAsync(&h[1], nrep, sizeof(int), cudaMemcpyDeviceToHost, st));
