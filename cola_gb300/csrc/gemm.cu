@@ -385,8 +385,8 @@ static int launch_tile(GemmArgs<T, S>& g, int split, bool xk, cudaStream_t st) {
   return launch_form<T, S, BM, BN, BK, WM, WN, WK, 2, false, false>(g, st);
 }
 
-// Tile choice.  Short FP32 sums (K <= 256: Kronecker factors above all) keep the plain order of k, one
-// warp group and no split: 48 or 64 rows x 128 columns, whichever pads M less, while that gives every SM a
+// Tile choice.  Short FP32 sums (K <= 256, and K <= 1024 where the caller asks for it: Kronecker factors, whose
+// products feed Lanczos recurrences) keep the plain order of k, one warp group and no split: 48 or 64 rows x 128 columns, whichever pads M less, while that gives every SM a
 // tile, else 32 x 32 (32 x 16 for few columns).  Longer sums: 64 x 64 while that gives every SM a tile, else
 // the column tile that N fills, with clusters along k until the grid covers 1.5 times the SMs and each
 // CTA keeps at least two k-slices.  Measured (FP32, back-to-back launches, which cost 6.2 us for the
@@ -395,7 +395,7 @@ static int launch_tile(GemmArgs<T, S>& g, int split, bool xk, cudaStream_t st) {
 // 12.4 us (16.5 us in 64-row tiles); 128 x 128 x 2048 8.2 us; 64 x 64 x 262,144 84 us.
 template <class T, class S>
 int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, int64_t x_p, int64_t x_k, T* Y,
-                   int64_t y_p, int64_t y_m, int64_t P, int64_t q, T alpha, T beta, const int* skip,
+                   int64_t y_p, int64_t y_m, int64_t P, int64_t q, T alpha, T beta, bool plain, const int* skip,
                    cudaStream_t st) {
   GemmArgs<T, S> g;
   g.A = A; g.lda = lda; g.M = M; g.K = K;
@@ -419,7 +419,7 @@ int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, in
     return s;
   };
   if constexpr (std::is_same<T, float>::value) {
-    if (K <= 256) {
+    if (K <= 256 || (plain && K <= 1024)) {
       const bool b48 = ceil_div(M, 48) * 48 < ceil_div(M, 64) * 64;
       if (b48 && tiles(48, 128) >= sms) return launch_tile<T, S, 48, 128, 16, 2, 2, 1, 3>(g, 1, xk, st);
       if (!b48 && tiles(64, 128) >= sms) return launch_tile<T, S, 64, 128, 16, 2, 2, 1, 3>(g, 1, xk, st);
@@ -440,7 +440,7 @@ int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, in
 
 #define COLAGB_INST(T, S)                                                                                         \
   template int dense_contract<T, S>(const S*, int64_t, int64_t, int64_t, const T*, int64_t, int64_t, T*, int64_t, \
-                                    int64_t, int64_t, int64_t, T, T, const int*, cudaStream_t);
+                                    int64_t, int64_t, int64_t, T, T, bool, const int*, cudaStream_t);
 COLAGB_INST(float, float)
 COLAGB_INST(float, __nv_bfloat16)
 COLAGB_INST(double, double)

@@ -399,7 +399,8 @@ static int launch_dense(const colagb_op_node& nd, const T* X, int64_t ldx, int64
       default: dense_gemv_kernel<T, S, 4><<<grid, 256, 0, st>>>(A, nd.ld, nd.rows, nd.cols, X, ldx, bsx, Y, ldy, bsy, alpha, beta, skip); break;
     }
   } else {
-    return dense_contract<T, S>(A, nd.ld, nd.rows, nd.cols, X, bsx, ldx, Y, bsy, ldy, batch, k, alpha, beta, skip, st);
+    return dense_contract<T, S>(A, nd.ld, nd.rows, nd.cols, X, bsx, ldx, Y, bsy, ldy, batch, k, alpha, beta, false,
+                                skip, st);
   }
   COLAGB_CUDA(cudaGetLastError());
   return COLAGB_OK;
@@ -512,7 +513,7 @@ static int contract_leaf(const colagb_op_node& f, const T* X, int64_t x_p, int64
                          int64_t P, int64_t q, T alpha, T beta, const int* skip, cudaStream_t st) {
 #define COLAGB_CONTRACT(S)                                                                                        \
   return dense_contract<T, S>(static_cast<const S*>(f.data), f.ld, f.rows, f.cols, X, x_p, x_k, Y, y_p, y_m, P, q, \
-                              alpha, beta, skip, st)
+                              alpha, beta, true, skip, st)
   if (f.dtype == COLAGB_F32) COLAGB_CONTRACT(float);
   if (f.dtype == COLAGB_BF16) COLAGB_CONTRACT(__nv_bfloat16);
   if constexpr (std::is_same<T, double>::value) COLAGB_CONTRACT(double);

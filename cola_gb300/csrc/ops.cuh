@@ -29,10 +29,11 @@ int launch_axpby(const T* X, int64_t ldx, T* Y, int64_t ldy, int64_t rows, int64
                  const int* skip, cudaStream_t st);
 
 // Y[m, n] = alpha * sum_k A[m, k] X[k, n] + beta * Y[m, n] for the P * q columns n = (p, j), X[k, n] at
-// X + p x_p + k x_k + j, Y[m, n] at Y + p y_p + m y_m + j (gemm.cu).
+// X + p x_p + k x_k + j, Y[m, n] at Y + p y_p + m y_m + j (gemm.cu).  plain: sums of up to 1024 FP32 terms are
+// taken in the plain order of k.
 template <class T, class S>
 int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, int64_t x_p, int64_t x_k, T* Y,
-                   int64_t y_p, int64_t y_m, int64_t P, int64_t q, T alpha, T beta, const int* skip,
+                   int64_t y_p, int64_t y_m, int64_t P, int64_t q, T alpha, T beta, bool plain, const int* skip,
                    cudaStream_t st);
 
 // Whether the operator is a single CSR or Dense leaf, optionally plus a scalar shift
