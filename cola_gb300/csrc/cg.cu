@@ -14,7 +14,8 @@
 // Two executions of that loop:
 //   * fused: one cooperative persistent kernel runs the whole solve for a Dense or CSR operator
 //     (optionally + c*I) with P = identity or Diagonal; three bounded grid barriers per step.
-//   * generic: any operator program / preconditioner; four launches per step, the stop test is
+//   * generic: any operator program / preconditioner; after the operator's launches one (short vectors, P =
+//     identity or Diagonal), three or more launches per step, the stop test is
 //     evaluated on the device and the host polls it every `check_every` steps (the reference
 //     syncs twice per step, torch_tqdm.py:42 and cg.py:136).
 // Column sums are reduced in a fixed order so every CTA derives bit-identical alpha / beta.
@@ -450,6 +451,206 @@ __global__ void k_pupdate(T* P, const T* R, const T* Z, const T* dinv, int64_t n
     const T z = PK == 0 ? r : (PK == 1 ? dinv[i] * r : Z[u]);
     P[u] = z + s.beta[c] * P[u];
   });
+}
+
+// One step after Ap in a single launch (P = identity or Diagonal), by one cluster of kTailCtas CTAs (Ap stands for
+// AP + shift p: the scalar part of A = B + c I is added here instead of by a launch of its own):
+//   <p, Ap>, alpha ; x += alpha p, r -= alpha Ap, |r|^2, <r, z>, beta, stop test ; p = z + beta p,
+// the CTAs' column sums added through distributed shared memory in rank order by every CTA.  For blocks of up
+// to kTailMax entries the step is bound by the launches and the last-block reductions of k_alpha, k_update
+// and k_pupdate (8 + 11 + 3 us at 7680 x 8, 2 us of which move the vectors); larger ones want all SMs.
+constexpr int kTailCtas = 16, kTailThreads = 1024;
+// (FP64: 16 SMs have 32 multiply-adds a cycle between them, six per entry.)
+template <class T> constexpr int64_t kTailMax = std::is_same<T, double>::value ? 48 * 1024 : 512 * 1024;
+constexpr int64_t kTailMaxCols = 512;
+
+// Column sums of the CTA, as block_col_sums, for the tail: with a power-of-two number of FP32 columns up to 32
+// the lanes of a column are added by shuffles and the warps in one more step (the general tree passes ten
+// block barriers for one column).
+template <int NQ, class T, class F>
+__device__ __forceinline__ void tail_col_sums(int64_t n, int64_t k, int rank, F f, T* const (&out)[NQ], T* smem) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (k <= 32 && (k & (k - 1)) == 0) {
+      const int t = threadIdx.x, lane = t & 31, warp = t >> 5, kc = (int)k, c = t & (kc - 1);
+      const int rpp = kTailThreads / kc;
+      T acc[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) acc[q] = T(0);
+      for (int64_t i = (int64_t)rank * rpp + t / kc; i < n; i += (int64_t)rpp * kTailCtas) f(i, c, acc);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        for (int o = 16; o >= kc; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+        if (lane < kc) smem[(q * 32 + lane) * 32 + warp] = acc[q];
+      }
+      __syncthreads();
+      for (int w = warp; w < NQ * kc; w += kTailThreads / 32) {  // warp w: value w / kc of column w % kc
+        const T v = warp_sum(smem[(w / kc * 32 + w % kc) * 32 + lane]);
+        if (lane == 0) out[w / kc][w % kc] = v;
+      }
+      __syncthreads();
+      return;
+    }
+  }
+  block_col_sums<NQ, T>(0, n, rank, kTailCtas, k, f, out, smem);
+}
+
+template <class T, int PK>
+__global__ void __launch_bounds__(kTailThreads, 1) k_cg_tail(T* X, int64_t ldx, T* R, T* P, const T* AP, T shift,
+                                                             const T* dinv, int64_t n, int64_t k, int max_iters, T* hist,
+                                                             CgScalars<T> s) {
+  if (*s.done) return;
+  namespace cgx = cooperative_groups;
+  cgx::cluster_group cl = cgx::this_cluster();
+  constexpr int NQ = PK == 1 ? 2 : 1;
+  extern __shared__ __align__(16) unsigned char tail_smem[];
+  T* const red = reinterpret_cast<T*>(tail_smem);  // NQ * kTailThreads
+  T* const pa = red + NQ * kTailThreads;           // this CTA's column sums: <p, Ap>; |r|^2; <r, z>
+  T* const pc = pa + k;
+  T* const pb = pc + k;
+  T* const alpha = pb + k;
+  T* const beta = alpha + k;
+  __shared__ int s_any;
+  const int t = threadIdx.x, rank = (int)cl.block_rank();
+  // the state of this thread's column (k <= kTailThreads), read before the first cluster barrier: rank 0 may
+  // move it on after that
+  T gamma = T(0), rnorm = T(0), tol_eff = T(0);
+  if (t < k) {
+    gamma = s.gamma[t];
+    rnorm = s.rnorm[t];
+    tol_eff = s.tol_eff[t];
+  }
+  const int it = *s.iters + 1;
+  if (t == 0) s_any = 0;
+  T* const out_a[1] = {pa};
+  tail_col_sums<1, T>(n, k, rank,
+                      [&](int64_t i, int64_t c, T (&acc)[1]) {
+                        const T p = P[i * k + c];
+                        acc[0] += p * (AP[i * k + c] + shift * p);
+                      },
+                      out_a, red);
+  cl.sync();
+  const bool conv = rnorm < SmallValue<T>::v;
+  if (t < k) {
+    T v[kTailCtas], tot = T(0);  // the peers' sums in flight together
+#pragma unroll
+    for (int q = 0; q < kTailCtas; ++q) v[q] = *cl.map_shared_rank(pa + t, q);
+#pragma unroll
+    for (int q = 0; q < kTailCtas; ++q) tot += v[q];
+    alpha[t] = conv ? T(0) : safe_div(gamma, tot);
+  }
+  __syncthreads();
+  T* out_c[NQ];
+  out_c[0] = pc;
+  if constexpr (NQ == 2) out_c[1] = pb;
+  T* const (&outs)[NQ] = out_c;
+  tail_col_sums<NQ, T>(n, k, rank,
+                       [&](int64_t i, int64_t c, T (&acc)[NQ]) {
+                         const T al = alpha[c], p = P[i * k + c];
+                         X[i * ldx + c] += al * p;
+                         const T r = R[i * k + c] - al * (AP[i * k + c] + shift * p);
+                         R[i * k + c] = r;
+                         acc[0] += r * r;
+                         if constexpr (NQ == 2) acc[1] += r * (dinv[i] * r);
+                       },
+                       outs, red);
+  cl.sync();
+  T rn = T(0), g1 = T(0);
+  if (t < k) {
+    T v[kTailCtas], w[kTailCtas], rr = T(0), rz = T(0);
+#pragma unroll
+    for (int q = 0; q < kTailCtas; ++q) {
+      v[q] = *cl.map_shared_rank(pc + t, q);
+      if constexpr (NQ == 2) w[q] = *cl.map_shared_rank(pb + t, q);
+    }
+#pragma unroll
+    for (int q = 0; q < kTailCtas; ++q) {
+      rr += v[q];
+      if constexpr (NQ == 2) rz += w[q];
+    }
+    g1 = NQ == 2 ? rz : rr;
+    beta[t] = conv ? T(0) : safe_div(g1, gamma);
+    rn = sqrt(rr);
+    if (rn > tol_eff) atomicOr(&s_any, 1);
+    if (rank == 0) pa[t] = rn;  // every peer has read its <p, Ap>
+  }
+  __syncthreads();
+  // the peers' sums are read: arrive now, wait at the end, so that no CTA leaves while another reads its
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  const bool done = !(s_any && it < max_iters);
+  if (!done) {  // p is not read after the last step
+    const int kc = (int)k, rpp = kTailThreads / kc, my_r = t / kc, c = t % kc;
+    if (my_r < rpp) {
+      const T be = beta[c];
+      for (int64_t i = (int64_t)rank * rpp + my_r; i < n; i += (int64_t)rpp * kTailCtas) {
+        const T r = R[i * k + c];
+        P[i * k + c] = (PK == 0 ? r : dinv[i] * r) + be * P[i * k + c];
+      }
+    }
+  }
+  if (rank == 0) {
+    if (t < k) {
+      s.gamma[t] = g1;
+      s.rnorm[t] = rn;
+    }
+    if (t == 0) {
+      *s.iters = it;
+      if (hist) {
+        T m = T(0);
+        for (int64_t c = 0; c < k; ++c) m += pa[c];
+        hist[it] = m / (T)k;
+      }
+      *s.done = done;
+    }
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+template <class T, int PK>
+static int launch_tail(T* X, int64_t ldx, T* R, T* P, const T* AP, T shift, const T* dinv, int64_t n, int64_t k,
+                       int max_iters, T* hist, const CgScalars<T>& s, cudaStream_t st) {
+  auto* f = k_cg_tail<T, PK>;
+  const size_t smem = sizeof(T) * ((PK == 1 ? 2 : 1) * kTailThreads + 5 * k);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kTailCtas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(kTailCtas);
+  cfg.blockDim = dim3(kTailThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  COLAGB_CUDA(cudaLaunchKernelEx(&cfg, f, X, ldx, R, P, AP, shift, dinv, n, k, max_iters, hist, s));
+  return COLAGB_OK;
+}
+
+// Whether the step's tail runs as one cluster here (sizes, and the device can schedule the cluster).
+template <class T, int PK>
+static bool tail_ok(int64_t n, int64_t k) {
+  if (n * k > kTailMax<T> || k > kTailMaxCols) return false;
+  auto* f = k_cg_tail<T, PK>;
+  const size_t smem = sizeof(T) * ((PK == 1 ? 2 : 1) * kTailThreads + 5 * k);
+  if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kTailCtas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(kTailCtas);
+  cfg.blockDim = dim3(kTailThreads);
+  cfg.dynamicSmemBytes = smem;
+  int ncl = 0;
+  if (cudaOccupancyMaxActiveClusters(&ncl, f, &cfg) != cudaSuccess) cudaGetLastError();
+  return ncl >= 1;
 }
 
 template <class T>
@@ -980,13 +1181,31 @@ static int run_generic(const colagb_op* A, const colagb_op* P, const CgPlan& pl,
   COLAGB_CUDA(cudaGetLastError());
   int h_done[2] = {0, 0};
   const int every = prm.check_every > 0 ? prm.check_every : 16;
+  const bool tail = pl.pk == 0 ? tail_ok<T, 0>(n, k) : pl.pk == 1 && tail_ok<T, 1>(n, k);
+  // the node whose product a step forms, and what the tail adds to it
+  int a_node = A->root;
+  T shift = T(0);
+  if (tail && A->nodes[a_node].kind == COLAGB_OP_SUM && A->children[a_node].size() == 2)
+    for (int e = 0; e < 2; ++e) {
+      const int other = A->children[A->root][1 - e];
+      const colagb_op_node& c = A->nodes[A->children[A->root][e]];
+      if (a_node == A->root && (c.kind == COLAGB_OP_SCALAR || c.kind == COLAGB_OP_IDENTITY)) {
+        shift = c.kind == COLAGB_OP_SCALAR ? (T)c.scalar : T(1);
+        a_node = other;
+      }
+    }
   // One step of the loop: Ap, alpha, x / r update (+ z = P r and gamma for a general P), p update.
   // Every kernel reads the device stop flag and does nothing once it is set, so a block of steps may
   // run past convergence or max_iters (the device counts the steps and enforces max_iters).
   auto enqueue_steps = [&](cudaStream_t q, int nsteps) -> int {
     for (int j = 0; j < nsteps; ++j) {
       Bump w(opws, opws_bytes);
-      COLAGB_TRY(op_apply<T>(A, A->root, Pv, k, 0, AP, k, 0, k, 1, T(1), T(0), w, s.done, q));
+      COLAGB_TRY(op_apply<T>(A, a_node, Pv, k, 0, AP, k, 0, k, 1, T(1), T(0), w, s.done, q));
+      if (tail) {
+        if (pl.pk == 0) COLAGB_TRY((launch_tail<T, 0>(X, ldx, R, Pv, AP, shift, dinv, n, k, prm.max_iters, hist, s, q)));
+        else COLAGB_TRY((launch_tail<T, 1>(X, ldx, R, Pv, AP, shift, dinv, n, k, prm.max_iters, hist, s, q)));
+        continue;
+      }
       k_alpha<T><<<nb, 256, 0, q>>>(Pv, AP, n, k, s);
       switch (pl.pk) {
         case 0: k_update<T, 0><<<nb, 256, 0, q>>>(X, ldx, R, Pv, AP, dinv, n, k, prm.max_iters, hist, s); break;

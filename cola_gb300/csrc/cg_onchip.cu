@@ -1241,36 +1241,53 @@ __global__ void __launch_bounds__(kST, 1) k_spare_pcg(const __grid_constant__ On
 }
 
 // ---- pattern analysis: the set of diagonals (column - row) a CSR pattern occupies ----
+// Nearly all entries repeat one of a few offsets: a CTA remembers those it has recorded in a small
+// direct-mapped table (an atomic per entry on the same few words took 526 us for 1.3M entries).
 __global__ void k_offset_bitmap(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t n,
                                 unsigned int* bits) {
+  __shared__ int64_t seen[256];
+  for (int t = threadIdx.x; t < 256; t += blockDim.x) seen[t] = -1;
+  __syncthreads();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     for (int32_t e = indptr[i]; e < indptr[i + 1]; ++e) {
       const int64_t o = (int64_t)indices[e] - i + (n - 1);  // [0, 2n - 2] for valid columns
-      if (o >= 0 && o < 2 * n - 1) atomicOr(bits + (o >> 5), 1u << (o & 31));
+      if (o < 0 || o >= 2 * n - 1) continue;
+      volatile int64_t* slot = seen + (((unsigned)o * 2654435761u) >> 24);
+      if (*slot == o) continue;
+      atomicOr(bits + (o >> 5), 1u << (o & 31));
+      *slot = o;
     }
 }
 
 // out[0] = number of distinct diagonals, out[1 .. 32] = the first 32 offsets in ascending order.
 __global__ void k_offset_collect(const unsigned int* __restrict__ bits, int64_t nwords, int64_t n, int* out) {
-  __shared__ int cnt[1024];
+  __shared__ int cnt[32];
   const int t = threadIdx.x;
   const int64_t per = (nwords + blockDim.x - 1) / blockDim.x;
   const int64_t w0 = t * per, w1 = (w0 + per < nwords) ? w0 + per : nwords;
   int c = 0;
   for (int64_t w = w0; w < w1; ++w) c += __popc(bits[w]);
-  cnt[t] = c;
+  // exclusive prefix of the counts: per warp, then over the warps (1024 threads)
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((t & 31) >= o) incl += v;
+  }
+  if ((t & 31) == 31) cnt[t >> 5] = incl;
   __syncthreads();
-  if (t == 0) {
-    int acc = 0;
-    for (int u = 0; u < (int)blockDim.x; ++u) {
-      const int v = cnt[u];
-      cnt[u] = acc;
-      acc += v;
+  if (t < 32) {
+    int w = t < (int)(blockDim.x >> 5) ? cnt[t] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, w, o);
+      if (t >= o) w += v;
     }
-    out[0] = acc;
+    cnt[t] = w;
+    if (t == 31) out[0] = w;
   }
   __syncthreads();
-  int rnk = cnt[t];
+  int rnk = incl - c + (t >= 32 ? cnt[(t >> 5) - 1] : 0);
   for (int64_t w = w0; w < w1 && rnk < 32; ++w) {
     unsigned int b = bits[w];
     while (b && rnk < 32) {

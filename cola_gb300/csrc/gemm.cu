@@ -45,6 +45,17 @@ struct GemmArgs {
   const int* skip;
 };
 
+// quotient and remainder of a column or tile index; 32-bit operands (nearly always) avoid the long division
+__device__ __forceinline__ void div_mod(int64_t a, int64_t b, int64_t& d, int64_t& m) {
+  if ((a | b) >> 32 == 0) {
+    d = (uint32_t)a / (uint32_t)b;
+    m = (uint32_t)a - (uint32_t)d * (uint32_t)b;
+  } else {
+    d = a / b;
+    m = a - d * b;
+  }
+}
+
 template <class T> __device__ __forceinline__ void ld_quad(const T* p, T v[4]);
 template <> __device__ __forceinline__ void ld_quad<float>(const float* p, float v[4]) {
   const float4 t = __ldg(reinterpret_cast<const float4*>(p));
@@ -115,7 +126,9 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) k_gemm(const __grid_constan
   const int ly = lane >> 3, lx = lane & 7;
   const int rank = (int)(blockIdx.x % (unsigned)g.split);
   const int64_t tid = blockIdx.x / (unsigned)g.split;
-  const int64_t m0 = (tid % g.mtiles) * BM, n0 = (tid / g.mtiles) * BN;
+  int64_t tile_n, tile_m;
+  div_mod(tid, g.mtiles, tile_n, tile_m);
+  const int64_t m0 = tile_m * BM, n0 = tile_n * BN;
   // this CTA's k range, in whole slices
   const int64_t slices = ceil_div(g.K, (int64_t)BK), per = ceil_div(slices, (int64_t)g.split);
   const int64_t s0 = rank * per < slices ? rank * per : slices;
@@ -139,8 +152,10 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) k_gemm(const __grid_constan
     const int nn = XK ? u / (BK / 4) : 4 * (u % (BN / 4)), kk = XK ? 4 * (u % (BK / 4)) : u / (BN / 4);
     xin[i] = u < XQ && n0 + nn < g.N;
     const int64_t n = xin[i] ? n0 + nn : 0;
-    px[i] = g.X + n / g.q * g.x_p + n % g.q + (s0 * BK + kk) * g.x_k;
-    left[i] = (int)(g.q - n % g.q < 4 ? g.q - n % g.q : 4);
+    int64_t p, j;
+    div_mod(n, g.q, p, j);
+    px[i] = g.X + p * g.x_p + j + (s0 * BK + kk) * g.x_k;
+    left[i] = (int)(g.q - j < 4 ? g.q - j : 4);
   }
   T ra[ASYNC ? 1 : NA][4], rx[ASYNC ? 1 : NX][4];
   auto fetch = [&](int64_t s, int b) {  // slice s: into buffer b (ASYNC) or into registers
@@ -267,8 +282,10 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) k_gemm(const __grid_constan
       }
       const T* as = smem + b * (LA + LX) + (wm * 4 * TM + ly) * PA + wk * KW;
       const T* xs = smem + b * (LA + LX) + LA + wk * KW * PX;
+      const int64_t kleft = g.K - (s0 + i) * BK - wk * KW;  // k-steps of this warp group that exist
 #pragma unroll
       for (int kq = 0; kq < KW; kq += 4) {
+        if (kq >= kleft) break;
         T av[TM][4];
 #pragma unroll
         for (int i = 0; i < TM; ++i) lds_quad(as + 4 * i * PA + kq, av[i]);
@@ -304,7 +321,9 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) k_gemm(const __grid_constan
     for (int j = 0; j < TN; ++j) {
       const int64_t n = n0 + col_of(j);
       if (n >= g.N) continue;
-      T* yc = g.Y + n / g.q * g.y_p + n % g.q;
+      int64_t p, jj;
+      div_mod(n, g.q, p, jj);
+      T* yc = g.Y + p * g.y_p + jj;
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
         const int64_t m = m0 + wm * 4 * TM + ly + 4 * i;
@@ -344,7 +363,9 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) k_gemm(const __grid_constan
     } else {
       for (int r = 0; r < g.split; ++r) sum += *cl.map_shared_rank(&tile[mm * BN + nn], r);
     }
-    T* y = g.Y + n / g.q * g.y_p + m * g.y_m + n % g.q;
+    int64_t p, j;
+    div_mod(n, g.q, p, j);
+    T* y = g.Y + p * g.y_p + m * g.y_m + j;
     *y = g.beta == T(0) ? g.alpha * sum : g.alpha * sum + g.beta * (*y);
   }
   if (g.split > 1) cl.sync();  // no CTA leaves while a peer may still read its tile
@@ -432,9 +453,11 @@ int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, in
     if (g.N > 8) return launch_tile<T, S, 32, 16, 32, 1, 1, 4, 4>(g, split_for(32, 16, 32), xk, st);
     return launch_tile<T, S, 32, 8, 64, 1, 1, 4, 4>(g, split_for(32, 8, 64), xk, st);
   } else {
-    if (g.N > 16 && tiles(32, 32) >= sms) return launch_tile<T, S, 32, 32, 16, 1, 1, 4, 4>(g, split_for(32, 32, 16), xk, st);
-    if (g.N > 8) return launch_tile<T, S, 32, 16, 32, 1, 1, 4, 4>(g, split_for(32, 16, 32), xk, st);
-    return launch_tile<T, S, 32, 8, 32, 1, 1, 4, 4>(g, split_for(32, 8, 32), xk, st);
+    // FP64 multiply-adds are the bound (80 cycles of a scheduler per warp instruction, padding included):
+    // the largest tile that gives every scheduler two warps, else 16 x 8
+    if (g.N > 16 && tiles(32, 32) >= 2 * sms) return launch_tile<T, S, 32, 32, 16, 1, 1, 4, 4>(g, 1, xk, st);
+    if (g.N > 8 && tiles(32, 16) >= 2 * sms) return launch_tile<T, S, 32, 16, 32, 1, 1, 4, 4>(g, 1, xk, st);
+    return launch_tile<T, S, 16, 8, 32, 1, 1, 4, 4>(g, split_for(16, 8, 32), xk, st);
   }
 }
 
