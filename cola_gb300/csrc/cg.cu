@@ -458,7 +458,7 @@ __global__ void k_pupdate(T* P, const T* R, const T* Z, const T* dinv, int64_t n
 //   <p, Ap>, alpha ; x += alpha p, r -= alpha Ap, |r|^2, <r, z>, beta, stop test ; p = z + beta p,
 // the CTAs' column sums added through distributed shared memory in rank order by every CTA.  For blocks of up
 // to kTailMax entries the step is bound by the launches and the last-block reductions of k_alpha, k_update
-// and k_pupdate (8 + 11 + 3 us at 7680 x 8, 2 us of which move the vectors); larger ones want all SMs.
+// and k_pupdate (8.3 + 11.5 + 3.4 us at 7680 x 8, here 9.7 us); larger ones want all SMs.
 constexpr int kTailCtas = 16, kTailThreads = 1024;
 // (FP64: 16 SMs have 32 multiply-adds a cycle between them, six per entry.)
 template <class T> constexpr int64_t kTailMax = std::is_same<T, double>::value ? 48 * 1024 : 512 * 1024;
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_cg_tail(T* X, int64_t ldx, 
   }
   __syncthreads();
   // the peers' sums are read: arrive now, wait at the end, so that no CTA leaves while another reads its
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
   const bool done = !(s_any && it < max_iters);
   if (!done) {  // p is not read after the last step
     const int kc = (int)k, rpp = kTailThreads / kc, my_r = t / kc, c = t % kc;
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_cg_tail(T* X, int64_t ldx, 
       *s.done = done;
     }
   }
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
 }
 
 template <class T, int PK>

