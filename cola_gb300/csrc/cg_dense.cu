@@ -21,7 +21,7 @@
 // The schedules before: 16 CTAs in one cluster for matrices up to 32 MB, which two cluster reductions, a
 // third barrier and 1 MB of L2 reads per CTA held at 12.9 us a step for 2048 x 2048 FP32 and 19.5 us for
 // 200 x 200 FP64; several right-hand sides read the matrix once each (111 us for 3001 x 3001 BF16 x 3).
-// Now 4.4, 5.3 and 11.5 us; what is left is the barrier (1.3 us), the L2 round trips around it and the
+// Now 4.6, 5.3 and 11.5 us; what is left is the barrier (1.3 us), the L2 round trips around it and the
 // two block sums, in FP64 also the divisions and adds themselves (64 cycles of a scheduler each).
 #include <cooperative_groups.h>
 
@@ -130,9 +130,16 @@ __device__ __forceinline__ void dc_rows(const S* A, int64_t lda, int R, int n, i
   const int U = (np + 127) / 128;
   constexpr int V = RB * K, LV = ilog2(V);
   for (int rb = wr * RB; rb < R; rb += WR * RB) {
-    T acc[V];
+    // one FP32 column, streamed rows: a lane's sum in pieces of 32 terms (one chain of 172 at n = 5500 left the
+    // solution 1.25 times further from the exact one).  Rows that fit shared memory are short enough without.
+    constexpr bool PIECES = std::is_same<T, float>::value && K == 1 && FORM != 0;
+    T acc[V], total[PIECES ? V : 1];
 #pragma unroll
-    for (int i = 0; i < V; ++i) acc[i] = T(0);
+    for (int i = 0; i < V; ++i) {
+      acc[i] = T(0);
+      if constexpr (PIECES) total[i] = T(0);
+    }
+    int left = 8;
     const S* row[RB];  // rows beyond R repeat the last one; their sums are not stored
 #pragma unroll
     for (int i = 0; i < RB; ++i) row[i] = A + (int64_t)(rb + i < R ? rb + i : R - 1) * lda;
@@ -164,7 +171,19 @@ __device__ __forceinline__ void dc_rows(const S* A, int64_t lda, int R, int n, i
 #pragma unroll
           for (int e = 0; e < 4; ++e) acc[i * K + c] += a[i][e] * x[e];
       }
+      if constexpr (PIECES)
+        if (--left == 0) {
+          left = 8;
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            total[i] += acc[i];
+            acc[i] = T(0);
+          }
+        }
     }
+    if constexpr (PIECES)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] += total[i];
     const T s = warp_sum_many<V, T>(acc);
     const int id = lane >> (5 - LV);
     if ((lane & ((32 >> LV) - 1)) == 0 && rb + id / K < R) part[((size_t)wc * R + rb) * K + id] = s;
