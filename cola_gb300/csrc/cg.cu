@@ -12,8 +12,9 @@
 // Divisions use do_safe_div (:173-178): |denominator| < 1e-40 is replaced by 1e-40.
 //
 // Two executions of that loop:
-//   * fused: one cooperative persistent kernel runs the whole solve for a Dense or CSR operator
-//     (optionally + c*I) with P = identity or Diagonal; three bounded grid barriers per step.
+//   * fused: one persistent kernel runs the whole solve for a Dense or CSR operator (optionally + c*I) with
+//     P = identity or Diagonal: cg_dense.cu (k <= 8, one exchange per step) and cg_csr.cu (k = 1, two bounded
+//     grid barriers), else k_cg_fused below (CSR with k > 1, what the two do not hold; three barriers).
 //   * generic: any operator program / preconditioner; after the operator's launches one (short vectors, P =
 //     identity or Diagonal), three or more launches per step, the stop test is
 //     evaluated on the device and the host polls it every `check_every` steps (the reference
@@ -1296,8 +1297,9 @@ static int finish_fused(const CgScalars<T>& s, colagb_cg_result* res, cudaStream
 
 template <class T, class S, int PK>
 static int run_fused(const CgPlan& pl, const T* B, int64_t ldb, T* X, int64_t ldx, const colagb_cg_params& prm, T* hist,
-                     CgScalars<T> s, T* R, T* Pv, T* AP, colagb_cg_result* res, cudaStream_t st) {
+                     CgScalars<T> s, T* R, T* Pv, T* AP, colagb_cg_result* res, cudaStream_t st, bool* taken) {
   const colagb_op_node* leaf = pl.ff.leaf;
+  *taken = true;
   if constexpr (!(std::is_same<T, double>::value && std::is_same<S, __nv_bfloat16>::value))
   if (leaf->kind == COLAGB_OP_DENSE && pl.n <= (1 << 20)) {
     DenseCgArgs<T, S> d;
@@ -1324,6 +1326,14 @@ static int run_fused(const CgPlan& pl, const T* B, int64_t ldb, T* X, int64_t ld
     bool ran = false;
     COLAGB_TRY((cg_dense_solve<T, S>(d, st, &ran)));
     if (ran) return finish_fused(s, res, st);
+    // Several columns whose vectors do not fit its shared memory: the generic loop, whose product reads each
+    // row once for all columns (us a step, k_cg_fused -> generic with plain launches: 2300 x 8 FP32 414 -> 23,
+    // 6000 x 3 101 -> 76, 9001 x 2 82 -> 82, 20000 x 8 3573 -> 372, 1500 x 8 FP64 375 -> 60, 3000 x 8 BF16
+    // 649 -> 36; no measured size was slower).
+    if (pl.k > 1 && pl.n >= 8) {
+      *taken = false;
+      return COLAGB_OK;
+    }
   }
   if (leaf->kind == COLAGB_OP_CSR && pl.k == 1 && pl.n < ((int64_t)1 << 31) - 1) {
     CsrCgArgs<T, S> d;
@@ -1454,16 +1464,18 @@ static int cg_solve_t(const colagb_op* A, const colagb_op* P, const void* Bv, in
     res->status = COLAGB_OK;
     return COLAGB_OK;
   }
+  colagb_cg_params gp = prm;
   if (prm.allow_fused && pl.fused_ok) {
-    const int sd = pl.ff.leaf->dtype;
-    if (sd == COLAGB_BF16) {
-      return pl.pk == 0 ? run_fused<T, __nv_bfloat16, 0>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st)
-                        : run_fused<T, __nv_bfloat16, 1>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st);
-    }
-    return pl.pk == 0 ? run_fused<T, T, 0>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st)
-                      : run_fused<T, T, 1>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st);
+    const bool bf = pl.ff.leaf->dtype == COLAGB_BF16;
+    bool taken = false;
+    if (bf && pl.pk == 0) COLAGB_TRY((run_fused<T, __nv_bfloat16, 0>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st, &taken)));
+    else if (bf) COLAGB_TRY((run_fused<T, __nv_bfloat16, 1>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st, &taken)));
+    else if (pl.pk == 0) COLAGB_TRY((run_fused<T, T, 0>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st, &taken)));
+    else COLAGB_TRY((run_fused<T, T, 1>(pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, res, st, &taken)));
+    if (taken) return COLAGB_OK;
+    gp.graph = 1;  // plain launches, 4.5 us a step more: these calls never allocated for a graph
   }
-  return run_generic<T>(A, P, pl, B, ldb, X, ldx, prm, hist, s, R, Pv, AP, Z, opws, opws_b, res, st);
+  return run_generic<T>(A, P, pl, B, ldb, X, ldx, gp, hist, s, R, Pv, AP, Z, opws, opws_b, res, st);
 }
 
 }  // namespace colagb

@@ -138,7 +138,7 @@ typedef struct colagb_cg_params {
   double tol;            /* CG(tol=...) */
   int32_t max_iters;     /* CG(max_iters=...) */
   int32_t check_every;   /* host polls the device stop flag every this many iterations (0 = 16) */
-  int32_t allow_fused;   /* 1: use the single-launch persistent kernel when the operator allows it */
+  int32_t allow_fused;   /* 1: use a single-launch persistent kernel where operator and sizes allow it */
   int32_t graph;         /* multi-launch loop: 0 = capture one block of check_every steps as a CUDA graph
                             and replay it (when max_iters >= 2 * check_every); 1 = plain launches */
   int64_t spin_limit;    /* grid-barrier spin bound of the persistent kernel (0 = default) */

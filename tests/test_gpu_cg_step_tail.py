@@ -48,3 +48,29 @@ def test_step_tail(dtype, n1, n2, k, kind):
     general = cola.Product(cola.Diagonal(d), one) if kind == "jacobi" else cola.Product(one, one)
     y, info2 = cg(cola.PSD(op), b, P=general, tol=TOL[dtype], max_iters=400)
     assert abs(info["iterations"] - info2["iterations"]) <= 2
+
+
+@pytest.mark.parametrize("dtype,n,k,fused", [(torch.float32, 2150, 8, True), (torch.float32, 2250, 8, False),
+                                             (torch.float32, 2251, 5, False), (torch.bfloat16, 2400, 5, False),
+                                             (torch.float64, 1201, 8, False)])
+@pytest.mark.parametrize("form", ["plain", "jacobi_shift"])
+def test_dense_columns_that_do_not_fit(dtype, n, k, fused, form):
+    """Several columns beyond the one-exchange kernel's shared memory: the generic loop, without a graph.
+    Cond 5 (BF16 storage moves the eigenvalues by less than 5 * 2^-8 * 2)."""
+    vec = torch.float64 if dtype == torch.float64 else torch.float32
+    A = _factor(n, dtype, 7)
+    A = torch.tril(A) + torch.tril(A, -1).T
+    b = torch.randn(n, k, generator=torch.Generator().manual_seed(k), dtype=torch.float64).to("cuda", vec)
+    D, shift, P = cola.Dense(A), 0.0, None
+    op = D
+    if form == "jacobi_shift":
+        shift, op = 0.25, D + 0.25 * cola.I_like(D)
+        P = cola.Diagonal((1.0 / (A.diagonal().double() + 0.25)).to(vec))
+    tol = TOL[vec]
+    x, info = cg(cola.PSD(op), b, P=P, tol=tol, max_iters=400)
+    assert info["fused"] == fused and not info["graph"] and info["iterations"] - 1 <= 200
+    R = b.double() - A.double() @ x.double() - shift * x.double()
+    assert float((R.norm(dim=0) / b.double().norm(dim=0)).max()) <= 2 * tol + 200 * 25 * U[vec]
+    y, info2 = cg(cola.PSD(op), b, P=P, tol=tol, max_iters=400, allow_fused=False)
+    assert abs(info["iterations"] - info2["iterations"]) <= 2
+    assert len(info["errors"]) in (info["iterations"] - 1, info["iterations"])
