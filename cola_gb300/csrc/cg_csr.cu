@@ -277,10 +277,6 @@ __global__ void __launch_bounds__(NT, 1) k_cg_csr(const __grid_constant__ CsrCgA
     return dot;
   };
   const T tiny = std::is_same<T, float>::value ? T(0) : T(1e-80);  // |r| < 1e-40 <=> |r|^2 <= tiny
-  auto above = [&](T rr, T tol_eff) {  // |r| > tol_eff, without the root unless equal to rounding
-    const T t2 = tol_eff * tol_eff, u = std::is_same<T, float>::value ? T(1e-6f) : T(1e-14);
-    return rr > t2 + u * t2 ? true : rr < t2 - u * t2 ? false : sqrt(rr) > tol_eff;
-  };
 
   // mult = |b| ; x0 published through Z (and the previous p = 0) for the first product
   T q1[1] = {T(0)};
@@ -321,7 +317,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_csr(const __grid_constant__ CsrCgA
     const T rn = sqrt(rr);
     tol_eff = (T)a.tol * rn + (T)a.tol;
     if (b == 0 && t == 0 && a.hist) a.hist[0] = rn;
-    if (t == 0) s_run = above(rr, tol_eff) && it < a.max_iters;
+    if (t == 0) s_run = norm_above(rr, tol_eff) && it < a.max_iters;
   }
   // p of the step before, by parity: zero before the first one
   for (int i = t; i < R; i += NT) po[i] = T(0);
@@ -410,7 +406,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_csr(const __grid_constant__ CsrCgA
       rr = q2[0];
       bnew = conv ? T(0) : cs_safe_div(q2[1], gamma);
       gamma = q2[1];
-      if (t == 0) s_run = above(rr, tol_eff) && it < a.max_iters;
+      if (t == 0) s_run = norm_above(rr, tol_eff) && it < a.max_iters;
       // off the other CTAs' path: the last owning warp of the last CTA writes the history
       if (b == nb - 1 && t == OT - 1 && a.hist) a.hist[it] = sqrt(rr);
     }

@@ -340,16 +340,11 @@ __global__ void __launch_bounds__(kDcThreads, 1) k_cg_dense(const __grid_constan
   auto m_of = [&](int i, int e) -> T { return a.dinv ? (i + e < n ? a.dinv[i + e] : T(0)) : T(1); };
   const T tiny = std::is_same<T, float>::value ? T(0) : T(1e-80);  // |r| < 1e-40 <=> |r|^2 <= tiny
   T gamma[K], tol_eff[K], rr[K];
-  // |r| > tol_eff for any column, without the square root unless the two are equal to rounding
-  auto above = [&]() {
+  auto above = [&]() {  // for any column
     bool any = false;
-    const T u = std::is_same<T, float>::value ? T(1e-6f) : T(1e-14);
 #pragma unroll
     for (int c = 0; c < K; ++c)
-      if (c < k) {
-        const T t2 = tol_eff[c] * tol_eff[c];
-        any |= rr[c] > t2 + u * t2 ? true : rr[c] < t2 - u * t2 ? false : sqrt(rr[c]) > tol_eff[c];
-      }
+      if (c < k) any |= norm_above(rr[c], tol_eff[c]);
     return any;
   };
   int it = 0;
