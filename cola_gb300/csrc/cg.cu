@@ -633,8 +633,8 @@ static bool tail_ok(int64_t n, int64_t k) {
   if (n * k > kTailMax<T> || k > kTailMaxCols) return false;
   auto* f = k_cg_tail<T, PK>;
   const size_t smem = sizeof(T) * ((PK == 1 ? 2 : 1) * kTailThreads + 5 * k);
-  if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  static_assert(sizeof(T) * (2 * kTailThreads + 5 * kTailMaxCols) <= 48 * 1024, "above the default limit");
+  if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kBT, 1) k_block_ir(const BlockArgs a) {
   }
 }
 
-constexpr size_t kBlockRed = 2 * kBT * sizeof(float4);
+constexpr size_t kBlockRed = 2 * kBT * sizeof(float4), kBlockRows = 120 * 1024;
 
 int block_padded_width(int64_t k) {
   int kp = 4;
@@ -478,9 +478,9 @@ int block_pcg_solve(const colagb_batched_csr* A, const double* B, double* X, con
     a.max_sweeps = prm->max_sweeps;
     // r in shared memory where the rows' share is at most half of it: three of a step's vector streams less
     const size_t r_bytes = (size_t)ceil_div(n, (int64_t)nb) * kp * sizeof(float);
-    a.r_resident = r_bytes <= 120 * 1024;
+    a.r_resident = r_bytes <= kBlockRows;
     const size_t smem = kBlockRed + (a.r_resident ? r_bytes : 0);
-    COLAGB_CUDA(cudaFuncSetAttribute(k_block_ir, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    COLAGB_CUDA(set_smem_limit(k_block_ir, kBlockRed + kBlockRows));
     a.gb.arrivals = reinterpret_cast<unsigned long long*>(bar);
     a.gb.err = reinterpret_cast<int*>(bar + 2);
     a.gb.nblocks = (unsigned)nb;

@@ -424,7 +424,7 @@ template <class T, class S, int NT>
 static int cs_launch(CsrCgArgs<T, S>& a, int nb, cudaStream_t st, bool* ran) {
   auto* f = k_cg_csr<T, S, NT>;
   a.smem = kCsSmem;
-  COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem));
+  COLAGB_CUDA(set_smem_limit(f, kCsSmem));
   int occ = 0;
   COLAGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, NT, a.smem));
   if (occ < 1) return COLAGB_OK;

@@ -520,7 +520,7 @@ static int dc_launch(DenseCgArgs<T, S>& a, cudaStream_t st, bool* ran) {
   if (n >= kDcCluster && (size_t)n * n * sizeof(S) <= kDcClusterBytes<T> && cl_b + rows_b <= kDcSmem) {
     auto* f = k_cg_dense<T, S, K, true>;
     COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cl_b + rows_b)));
+    COLAGB_CUDA(set_smem_limit(f, kDcSmem));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -554,7 +554,7 @@ static int dc_launch(DenseCgArgs<T, S>& a, cudaStream_t st, bool* ran) {
   // rows streamed element by element: the whole CTA sweeps a row (4001 FP32: 10.4 us a step, 13.6 otherwise)
   if (!a.resident && !a.aligned)
     for (a.wc = 1; a.wc < kDcWarps && 2 * a.wc <= ceil_div(n, (int64_t)128);) a.wc *= 2;
-  COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  COLAGB_CUDA(set_smem_limit(f, kDcSmem));
   int occ = 0;
   COLAGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, kDcThreads, smem));
   if (occ < 1) return COLAGB_OK;

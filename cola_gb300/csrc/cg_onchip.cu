@@ -1406,7 +1406,7 @@ static const SpareStreams* spare_streams() {
 template <int CL, int G>
 static int launch_onchip(const OnchipArgs& a, size_t smem, cudaStream_t st) {
   auto kern = k_onchip_pcg<CL, G>;
-  COLAGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  COLAGB_CUDA(set_smem_limit(kern, kOnchipSmemMax));
   if (CL > 8) COLAGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -1434,7 +1434,7 @@ static int launch_onchip(const OnchipArgs& a, size_t smem, cudaStream_t st) {
 template <int CL, int G>
 static int onchip_active_clusters(size_t smem, int* nclusters) {
   auto kern = k_onchip_pcg<CL, G>;
-  COLAGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  COLAGB_CUDA(set_smem_limit(kern, kOnchipSmemMax));
   if (CL > 8) COLAGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];

@@ -28,6 +28,15 @@ int check_cuda(cudaError_t e, const char* what);
     if (_s != COLAGB_OK) return _s; \
   } while (0)
 
+// A kernel's dynamic shared memory limit belongs to the function, not to the launch, and host threads share
+// it: it is always raised to the same constant, the most that kernel takes at any size, and only the
+// launch carries its own size.  (Set to each call's size, a smaller solve on one thread made a larger
+// one's launch on another fail.)
+template <class F>
+inline cudaError_t set_smem_limit(F* f, size_t most) {
+  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 int num_sms();                 // SM count of the current device (cached per device)

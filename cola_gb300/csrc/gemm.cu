@@ -395,7 +395,7 @@ static int launch_form(GemmArgs<T, S>& g, cudaStream_t st) {
   constexpr int PA = BK + 16 / (int)sizeof(T), LX = (BK * (XK ? BN + 1 : BN) + 3) / 4 * 4;
   constexpr size_t stage_b = sizeof(T) * ST * (BM * PA + LX), tile_b = WK > 1 ? sizeof(T) * BM * BN : 0;
   constexpr size_t smem = stage_b > tile_b ? stage_b : tile_b;
-  if (smem > 48 * 1024) COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) COLAGB_CUDA(set_smem_limit(f, smem));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

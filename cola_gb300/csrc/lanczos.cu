@@ -718,6 +718,7 @@ struct LzForm {
   int64_t chunk = 0;
   size_t smem = 0;
 };
+constexpr size_t kLzRunSmem = 160 * 1024, kLzProj1Smem = 220 * 1024;
 static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, int64_t slots, LzForm& f) {
   const bool al = (uintptr_t)basis % 16 == 0;
   f.blocks = nb;
@@ -728,21 +729,21 @@ static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, int64_t sl
   if (step == 0) return COLAGB_OK;
   const int64_t chunk = ceil_div(f.chunk, step) * step;  // a whole number of 128-float warp steps
   size_t smem = (size_t)(chunk * bs) * sizeof(float);
-  if (smem > 160 * 1024) return COLAGB_OK;
+  if (smem > kLzRunSmem) return COLAGB_OK;
   if (bs == 1) {  // the single-vector form keeps the coefficients in shared memory, too
     smem += (size_t)slots * sizeof(float);
-    if (smem > 220 * 1024) return COLAGB_OK;
+    if (smem > kLzProj1Smem) return COLAGB_OK;
   }
   f.form = bs == 1 ? 0 : 1;
   f.chunk = chunk;
   f.blocks = (int)ceil_div(n, chunk);
   f.smem = smem;
   if (f.form == 0) {
-    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_proj1<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_proj1<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    COLAGB_CUDA(set_smem_limit(k_lz_proj1<0>, kLzProj1Smem));
+    COLAGB_CUDA(set_smem_limit(k_lz_proj1<1>, kLzProj1Smem));
   } else {
-    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_projq<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    COLAGB_CUDA(cudaFuncSetAttribute(k_lz_projq<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    COLAGB_CUDA(set_smem_limit(k_lz_projq<0>, kLzRunSmem));
+    COLAGB_CUDA(set_smem_limit(k_lz_projq<1>, kLzRunSmem));
   }
   return COLAGB_OK;
 }
@@ -1055,6 +1056,8 @@ __global__ void __launch_bounds__(256) k_lz_reduce_h(int nblk, int64_t bs, int64
   }
 }
 
+constexpr size_t kGsSmem = 200 * 1024;
+
 // Launch plan of k_lz_gs for one run of the method.
 struct GsPlan {
   int vec = 1, run = 0, blocks = 1;
@@ -1075,7 +1078,7 @@ static GsPlan gs_plan(const T* basis, int64_t n, int64_t bs, int max_blocks) {
   p.run = (int)(units * unit);
   p.blocks = (int)std::min<int64_t>(target, ceil_div(N, (int64_t)p.run));
   p.smem = (size_t)p.run * sizeof(T) + (size_t)kGsThreads * p.vec * sizeof(T);
-  if (p.smem > 200 * 1024) {
+  if (p.smem > kGsSmem) {
     p.staged = false;
     p.vec = 1;
     p.smem = (size_t)kGsThreads * sizeof(T);
@@ -1086,7 +1089,7 @@ static GsPlan gs_plan(const T* basis, int64_t n, int64_t bs, int max_blocks) {
 template <class T, int VEC, int MODE, bool STAGED>
 static int launch_gs_form(const GsPlan& p, const GsArgs<T>& a, cudaStream_t st) {
   auto* f = k_lz_gs<T, VEC, MODE, STAGED>;
-  if (p.smem > 48 * 1024) COLAGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  COLAGB_CUDA(set_smem_limit(f, kGsSmem));
   f<<<p.blocks, kGsThreads, p.smem, st>>>(a);
   return COLAGB_OK;
 }
@@ -1694,6 +1697,7 @@ __global__ void k_tridiag_rq(const R* A, const R* Bv, int64_t m, const R* evecs,
   if (den > 0.0) evals[sys * m + j] = (R)(num / den);
 }
 
+constexpr size_t kTriSmem = 200 * 1024;
 template <class R>
 static int tridiag_eig(const R* a, const R* b, int64_t m, int64_t batch, R* evals, R* first_row, R* evecs,
                        int32_t* status, cudaStream_t st, const char* name) {
@@ -1702,13 +1706,12 @@ static int tridiag_eig(const R* a, const R* b, int64_t m, int64_t batch, R* eval
   if (m * batch == 0) return COLAGB_OK;
   // two sweeps' rotations while they fit, else one's: the warps then wait for the sweep they finish
   const size_t smem1 = (size_t)m * (5 * sizeof(R) + sizeof(int)), smem2 = smem1 + (size_t)m * 2 * sizeof(R);
-  const int two = smem2 <= 200 * 1024;
+  const int two = smem2 <= kTriSmem;
   const size_t smem = two ? smem2 : smem1;
-  if (smem > 200 * 1024) return fail(COLAGB_ERR_INVALID, "tridiagonal eigensolver: m too large");
-  if (smem > 48 * 1024)
-    COLAGB_CUDA(cudaFuncSetAttribute(k_tridiag_ql<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > kTriSmem) return fail(COLAGB_ERR_INVALID, "tridiagonal eigensolver: m too large");
+  COLAGB_CUDA(set_smem_limit(k_tridiag_ql<R>, kTriSmem));
   const size_t smem_rot = (size_t)m * kRotRows * sizeof(R);
-  if (evecs && smem_rot <= 200 * 1024) {
+  if (evecs && smem_rot <= kTriSmem) {
     // eigenvectors: QL records its rotations (one thread generates them serially), then many CTAs
     // replay them on the rows of Z in shared memory; applying them to Z in global memory from the
     // same CTA, row per thread, cost ~95 % of the solve
@@ -1724,8 +1727,7 @@ static int tridiag_eig(const R* a, const R* b, int64_t m, int64_t batch, R* eval
     k_tridiag_ql<R><<<(unsigned)batch, 128, smem, st>>>(a, b, m, two, evals, first_row, nullptr, status, rec, rec_i,
                                                         rec_n, rec_perm, cap);
     COLAGB_CUDA(cudaGetLastError());
-    if (smem_rot > 48 * 1024)
-      COLAGB_CUDA(cudaFuncSetAttribute(k_tridiag_apply<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rot));
+    COLAGB_CUDA(set_smem_limit(k_tridiag_apply<R>, kTriSmem));
     k_tridiag_apply<R><<<dim3((unsigned)ceil_div(m, (int64_t)kRotRows), (unsigned)batch), kRotRows, smem_rot, st>>>(
         rec, rec_i, rec_n, rec_perm, m, cap, evecs);
     COLAGB_CUDA(cudaGetLastError());
