@@ -130,16 +130,13 @@ __device__ __forceinline__ void dc_rows(const S* A, int64_t lda, int R, int n, i
   const int U = (np + 127) / 128;
   constexpr int V = RB * K, LV = ilog2(V);
   for (int rb = wr * RB; rb < R; rb += WR * RB) {
-    // one FP32 column, streamed rows: a lane's sum in pieces of 32 terms (one chain of 172 at n = 5500 left the
-    // solution 1.25 times further from the exact one).  Rows that fit shared memory are short enough without.
-    constexpr bool PIECES = std::is_same<T, float>::value && K == 1 && FORM != 0;
-    T acc[V], total[PIECES ? V : 1];
+    // One FP32 column: a quad's four products are added to each other before they join the lane's sum, so that
+    // a lane's chain has a link per quad.  (A link per product, 32 of them at n = 2048, left the solutions at
+    // condition 100 1.15 times further from the exact ones.)
+    constexpr bool QUADS = std::is_same<T, float>::value && K == 1;
+    T acc[V];
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      acc[i] = T(0);
-      if constexpr (PIECES) total[i] = T(0);
-    }
-    int left = 8;
+    for (int i = 0; i < V; ++i) acc[i] = T(0);
     const S* row[RB];  // rows beyond R repeat the last one; their sums are not stored
 #pragma unroll
     for (int i = 0; i < RB; ++i) row[i] = A + (int64_t)(rb + i < R ? rb + i : R - 1) * lda;
@@ -167,23 +164,14 @@ __device__ __forceinline__ void dc_rows(const S* A, int64_t lda, int R, int n, i
           dc_quad<T, T>(p + c * np + j, x, false);
         }
 #pragma unroll
-        for (int i = 0; i < RB; ++i)
+        for (int i = 0; i < RB; ++i) {
+          T sum = QUADS ? T(0) : acc[i * K + c];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[i * K + c] += a[i][e] * x[e];
-      }
-      if constexpr (PIECES)
-        if (--left == 0) {
-          left = 8;
-#pragma unroll
-          for (int i = 0; i < V; ++i) {
-            total[i] += acc[i];
-            acc[i] = T(0);
-          }
+          for (int e = 0; e < 4; ++e) sum += a[i][e] * x[e];
+          acc[i * K + c] = QUADS ? acc[i * K + c] + sum : sum;
         }
+      }
     }
-    if constexpr (PIECES)
-#pragma unroll
-      for (int i = 0; i < V; ++i) acc[i] += total[i];
     const T s = warp_sum_many<V, T>(acc);
     const int id = lane >> (5 - LV);
     if ((lane & ((32 >> LV) - 1)) == 0 && rb + id / K < R) part[((size_t)wc * R + rb) * K + id] = s;
