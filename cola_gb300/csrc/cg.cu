@@ -1291,6 +1291,7 @@ static int finish_fused(const CgScalars<T>& s, colagb_cg_result* res, cudaStream
   res->fused = 1;
   res->graph = 0;
   res->status = h[1];
+  if (h[1] == kCsrLeft) return COLAGB_OK;
   if (h[1] != 0) return fail(COLAGB_ERR_TIMEOUT, "fused CG: a grid barrier timed out");
   return COLAGB_OK;
 }
@@ -1357,11 +1358,13 @@ static int run_fused(const CgPlan& pl, const T* B, int64_t ldb, T* X, int64_t ld
     d.iters = s.iters;
     d.count = s.counters + 4;
     d.err = reinterpret_cast<int*>(s.counters + 6);
+    d.votes = s.counters + 7;
     d.spin_limit = prm.spin_limit > 0 ? prm.spin_limit : kDefaultSpinLimit;
     COLAGB_CUDA(cudaMemsetAsync(s.counters, 0, 8 * sizeof(unsigned int), st));
     bool ran = false;
     COLAGB_TRY((cg_csr_solve<T, S>(d, leaf->nnz, st, &ran)));
-    if (ran) return finish_fused(s, res, st);
+    if (ran) COLAGB_TRY(finish_fused(s, res, st));
+    if (ran && res->status != kCsrLeft) return COLAGB_OK;
   }
   FusedArgs<T, S> a;
   a.kind = leaf->kind;

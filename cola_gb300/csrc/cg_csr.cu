@@ -138,6 +138,10 @@ __global__ void __launch_bounds__(NT, 1) k_cg_csr(const __grid_constant__ CsrCgA
   const int w0 = s_lo, W = s_hi - s_lo;
   const bool window = used + (size_t)W * sizeof(T) <= (size_t)a.smem;
   T* const pw = reinterpret_cast<T*>(cs_smem + used);
+  bool too_long = false;
+  for (int i = t; i < R; i += NT) too_long |= rp[i + 1] - rp[i] > a.longest;
+  too_long = __syncthreads_or(too_long);
+  if (t == 0 && (too_long || !window)) atomicAdd(a.votes, too_long ? (unsigned)nb + 1 : 1u);  // gathers <= nb
 
   // arrive, wait for all CTAs; false when the wait gave up here or elsewhere
   auto barrier = [&]() -> bool {
@@ -291,6 +295,10 @@ __global__ void __launch_bounds__(NT, 1) k_cg_csr(const __grid_constant__ CsrCgA
   }
   publish(q1);
   if (!barrier()) return;
+  if (__ldcg(a.votes) > (unsigned)a.gathers) {  // every vote was cast before the barrier: all CTAs leave
+    if (b == 0 && t == 0) *a.err = kCsrLeft;
+    return;
+  }
   totals(q1);
   const T mult = share(owner ? sqrt(q1[0]) : T(0));
   if (window)
@@ -442,6 +450,21 @@ int cg_csr_solve(CsrCgArgs<T, S>& a, int64_t nnz, cudaStream_t st, bool* ran) {
   // a thread takes a row: rows longer than about 32 entries on average, and vectors too long for shared
   // memory beside a window of the same order, stay with the general kernel
   if (nnz > (int64_t)32 * a.n || own > (size_t)kCsSmem * 3 / 4) return COLAGB_OK;
+  // So do, us a step (general kernel / here, with Jacobi):
+  // short FP32 vectors, whose step is one cluster's three hardware barriers there and two software ones here:
+  // 64 unknowns per side 2-D 8.4 / 9.5, 90 9.1 / 9.4, 100 11.7 / 9.3; rows of 21 entries or more 12.0 / 11.1;
+  if (std::is_same<T, float>::value && a.n <= 8192 && nnz <= (int64_t)16 * a.n) return COLAGB_OK;
+  // matrices above 32 MB, which that kernel too spreads over all SMs (up to 32 MB it is one cluster), when
+  // their rows stream past a small L1 here: 15 random entries a row, n = 300,000 FP32 64 / 91, 21 in FP64
+  // 82 / 161, 31 within 5,000 columns, n = 100,000 FP64 52 / 83; 27-point 64^3 FP32 48 / 73; but 7 random entries,
+  // n = 600,000 FP32 86 / 73, 9-point 900^2 74 / 27, 15 near the diagonal, n = 600,000 FP32 64 / 57, 27-point 48^3
+  // FP64 (36 MB) 51 / 44;
+  const double mb = (double)nnz * (sizeof(S) + 4) / (1024 * 1024);
+  if ((mb > 48 && nnz > (int64_t)18 * a.n) || (mb > 32 && nnz > (int64_t)28 * a.n)) return COLAGB_OK;
+  a.gathers = mb <= 32 || nnz <= (int64_t)8 * a.n ? nb : nb / 8;  // a few: the ends of a periodic grid
+  // and rows of many entries, which one thread walks in both kernels: one full row, FP32 n = 30,000
+  // 2193 / 1826, 100,000 7275 / 10950; FP64 n = 50 26 / 20, 500 81 / 90, 30,000 3692 / 8360.
+  a.longest = std::is_same<T, float>::value ? 32768 : 256;
   // FP64: with few rows a CTA the 128 summing threads do everything (us a step with Jacobi, 128 / 512 threads:
   // 576 unknowns 8.6 / 10.0, 16,384 8.8 / 10.2, 65,536 11.7 / 11.6, 90,000 14.5 / 12.4, 262,144 23.1 / 18.1)
   if constexpr (std::is_same<T, double>::value)

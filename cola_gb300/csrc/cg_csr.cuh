@@ -27,7 +27,14 @@ struct CsrCgArgs {
   int* err;
   long long spin_limit;
   int smem;         // set by the launch: dynamic shared memory bytes
+  int gathers;      // set by the launch: the most CTAs that may lack a column window
+  int longest;      // set by the launch: the most entries of a row
+  unsigned int* votes;  // CTAs against taking the solve, zero at launch
 };
+
+// In *err: the CTAs left after the first barrier because of the pattern (a row longer than `longest`, or more
+// than `gathers` CTAs whose columns are too far apart for a window); x is untouched, the general kernel takes it.
+constexpr int kCsrLeft = -1;
 
 // CTAs a solve uses (the caller provides 4 partials for each).
 int cg_csr_blocks(int64_t n);
