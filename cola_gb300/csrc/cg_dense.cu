@@ -538,6 +538,12 @@ static int dc_launch(DenseCgArgs<T, S>& a, cudaStream_t st, bool* ran) {
   if (smem > kDcSmem) return COLAGB_OK;  // vectors too long: the general kernel
   a.resident = smem + rows_b <= kDcSmem;
   if (a.resident) smem += rows_b;
+  // Vectors above 195 KB leave half the L1 for the rows that stream past them (us a step at n = 16,000, 16,200 and
+  // 17,000, FP32: 168, 223 and 243).  One aligned FP32 column without Jacobi is faster on the general kernel then
+  // (192 and 195); with Jacobi (411 and 407 there), other types and more columns are not.
+  if (std::is_same<T, float>::value && std::is_same<S, float>::value && K == 1 && a.aligned && !a.dinv && !a.resident &&
+      smem > 195 * 1024)
+    return COLAGB_OK;
   dc_split<T, K>(n, (int)ceil_div(n, (int64_t)nb), &a.wc, &a.few);
   // rows streamed element by element: the whole CTA sweeps a row (4001 FP32: 10.4 us a step, 13.6 otherwise)
   if (!a.resident && !a.aligned)
