@@ -10,8 +10,9 @@
 // slots 1..i are visited here (same values, fewer bytes).
 //
 // Basis layout: slot j is an n x bs row-major block at basis + j*n*bs (probe index fastest), so
-// every pass reads contiguous, coalesced rows.  Per step: 1 operator application, 2 column-norm
-// reductions, 1 dot, and 2 x (V^T w then w -= V h) passes over the filled slots.
+// every pass reads contiguous, coalesced rows.  Per step: 1 operator application and 2 x (V^T w then w -= V h)
+// over the filled slots, with the norm summed in the last sweep and, in FP32, one dot and the three-term
+// update before; short vectors fuse a subtraction with the next projection, long ones take each as a pass.
 #include <cmath>
 #include <string>
 #include <vector>
@@ -55,6 +56,7 @@ __device__ __forceinline__ void lz_partials(int64_t n, int64_t bs, F f, T* out, 
     const int my_b = t % bc, my_r = t / bc;
     T acc = T(0);
     if (my_r < rpp)
+#pragma unroll 4
       for (int64_t r = (int64_t)blockIdx.x * rpp + my_r; r < n; r += (int64_t)rpp * gridDim.x) acc += f(r, b0 + my_b);
     smem[t] = acc;
     __syncthreads();
@@ -510,16 +512,70 @@ __global__ void __launch_bounds__(512, 2) k_lz_projq(const __grid_constant__ LzS
   }
 }
 
-// Any bs: a run is `chunk` rows.  Teams of 256 threads take four slots at a time (team q the groups q,
-// q + 4, ...); in a team, threads are rows x columns, w is read once for the four slots and the four
-// sums share one tree over the rows.
+// Partial projections of rows [r0, r1) on slots j0 .. j0 + 3 for j0 = first, first + stride, ... <= i, by 256 threads
+// (t of them, sync() their barrier, smem 4 x 256): threads are rows x columns, w is read once for four slots
+// and the four sums share one tree over the rows.
+constexpr int kLzTeam = 256, kLzSlots = 4;
+template <class T, int U, class Sync>
+__device__ __forceinline__ void lz_project_rows(const T* basis, const T* w, int64_t N, int64_t bs, int64_t r0, int64_t r1,
+                                                int first, int stride, int i, T* out, T* smem, int t, Sync sync) {
+  constexpr int JB = kLzSlots, TT = kLzTeam;
+  for (int64_t b0 = 0; b0 < bs; b0 += TT) {
+    const int bc = (int)((bs - b0) < TT ? (bs - b0) : TT);
+    const int rpp = TT / bc;
+    const int my_b = t % bc, my_r = t / bc;
+    for (int j0 = first; j0 <= i; j0 += stride) {
+      const int nj = (i - j0 + 1) < JB ? (i - j0 + 1) : JB;
+      T acc[JB] = {T(0), T(0), T(0), T(0)};
+      if (my_r < rpp) {
+        const T* v0 = basis + (int64_t)j0 * N + b0 + my_b;
+        // U rows' loads in flight together, the terms added in row order
+        for (int64_t r = r0 + my_r; r < r1; r += U * rpp) {
+          T wv[U], v[U][JB];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int64_t o = (r + u * rpp) * bs;
+            const bool in = r + u * rpp < r1;
+            wv[u] = in ? w[o + b0 + my_b] : T(0);
+#pragma unroll
+            for (int q = 0; q < JB; ++q) v[u][q] = in && q < nj ? v0[(int64_t)q * N + o] : T(0);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (r + u * rpp < r1) {
+#pragma unroll
+              for (int q = 0; q < JB; ++q) acc[q] = fma(v[u][q], wv[u], acc[q]);
+            }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < JB; ++q) smem[q * TT + t] = acc[q];
+      sync();
+      for (int wd = rpp; wd > 1;) {  // tree over the row slots, all JB sums at once
+        const int h = (wd + 1) >> 1;
+        if (my_r < wd - h) {
+#pragma unroll
+          for (int q = 0; q < JB; ++q) smem[q * TT + t] += smem[q * TT + t + h * bc];
+        }
+        sync();
+        wd = h;
+      }
+      if (t < bc) {
+        for (int q = 0; q < nj; ++q) out[(int64_t)(j0 + q) * bs + b0 + t] = smem[q * TT + t];
+      }
+      sync();
+    }
+  }
+}
+
+// Any bs, short vectors: a run is `chunk` rows; teams of 256 threads take four slots at a time (team q the
+// groups q, q + 4, ...).
 constexpr int kLzTeams = 4;
 template <int MODE>
 __global__ void __launch_bounds__(256 * kLzTeams) k_lz_projx(const __grid_constant__ LzStep a) {
   const LzState<float>& s = a.s;
   if (*s.done) return;
-  constexpr int JB = 4, TT = 256;
-  __shared__ float smem_all[kLzTeams * JB * TT];
+  __shared__ float smem_all[kLzTeams * kLzSlots * kLzTeam];
   const int i = *s.step;
   const int64_t n = a.n, bs = a.bs, N = n * bs;
   const int64_t r0 = (int64_t)blockIdx.x * a.chunk < n ? (int64_t)blockIdx.x * a.chunk : n;
@@ -533,44 +589,91 @@ __global__ void __launch_bounds__(256 * kLzTeams) k_lz_projx(const __grid_consta
       w[u] -= lz_comb1(a.basis, N, u, s.hbuf + b, bs, i);
   }
   __syncthreads();
-  const int team = threadIdx.x / TT, t = threadIdx.x % TT;
-  float* const smem = smem_all + team * JB * TT;
-  auto team_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(team + 1) : "memory"); };
-  float* out = s.hpart + (int64_t)blockIdx.x * a.slots * bs;
-  for (int64_t b0 = 0; b0 < bs; b0 += TT) {
-    const int bc = (int)((bs - b0) < TT ? (bs - b0) : TT);
-    const int rpp = TT / bc;
-    const int my_b = t % bc, my_r = t / bc;
-    for (int j0 = 1 + JB * team; j0 <= i; j0 += JB * kLzTeams) {
-      const int nj = (i - j0 + 1) < JB ? (i - j0 + 1) : JB;
-      float acc[JB] = {0.f, 0.f, 0.f, 0.f};
-      if (my_r < rpp) {
-        const float* v0 = a.basis + (int64_t)j0 * N + b0 + my_b;
-        for (int64_t r = r0 + my_r; r < r1; r += rpp) {
-          const float wv = w[r * bs + b0 + my_b];
-#pragma unroll
-          for (int q = 0; q < JB; ++q)
-            if (q < nj) acc[q] += v0[(int64_t)q * N + r * bs] * wv;
-        }
+  const int team = threadIdx.x / kLzTeam;
+  lz_project_rows<float, 1>(a.basis, w, N, bs, r0, r1, 1 + kLzSlots * team, kLzSlots * kLzTeams, i,
+                         s.hpart + (int64_t)blockIdx.x * a.slots * bs, smem_all + team * kLzSlots * kLzTeam,
+                         threadIdx.x % kLzTeam, [&]() { asm volatile("bar.sync %0, 256;" ::"r"(team + 1) : "memory"); });
+}
+
+// The same sums and updates as passes of their own, for long vectors: every pass then streams with all the
+// loads an SM can hold, where the fused kernels wait for one run at a time.  One CTA's run of rows is the
+// projx kernel's, so the sums are the same to the bit.
+template <class T>
+__global__ void __launch_bounds__(kLzTeam, 4) k_lz_project(const T* basis, const T* w, int64_t n, int64_t bs, int64_t slots,
+                                                        LzState<T> s) {
+  if (*s.done) return;
+  __shared__ T smem[kLzSlots * kLzTeam];
+  const int64_t chunk = ceil_div(n, (int64_t)gridDim.x);
+  const int64_t r0 = (int64_t)blockIdx.x * chunk < n ? (int64_t)blockIdx.x * chunk : n;
+  const int64_t r1 = r0 + chunk < n ? r0 + chunk : n;
+  // two rows at a time (one, at the compiler's choice: 2.4 instead of 0.95 ms for 64 columns of 1,000,000 FP32
+  // rows and 12 slots), within the 64 registers of four CTAs an SM
+  lz_project_rows<T, 2>(basis, w, n * bs, bs, r0, r1, 1, kLzSlots, *s.step, s.hpart + (int64_t)blockIdx.x * slots * bs, smem,
+                     threadIdx.x, []() { __syncthreads(); });
+}
+
+// w -= diag[i-1] V[i] + subdiag[i-1] V[i-1]
+__global__ void k_lz_terms(const __grid_constant__ LzStep a) {
+  if (*a.s.done) return;
+  const int i = *a.s.step;
+  const int64_t N = a.n * a.bs, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < N; u += step) {
+    const int64_t b = u % a.bs;
+    a.w[u] = lz_term(a.w[u], a.diag[b * a.max_iters + (i - 1)], a.vi[u], a.subdiag[b * (a.max_iters + 1) + (i - 1)], a.vim1[u]);
+  }
+}
+
+// w -= sum_j V[j] h[j], j = 1..i in order.  FORM 0: any bs; 1: float4 of blocks with bs % 4 == 0; 2: float4 of
+// one column.  The grid is eight CTAs an SM for the quads and four for single entries, of which a thread takes
+// four at a time; fewer loads in flight, or registers for fewer CTAs, were slower by up to two times.
+template <class T, int FORM>
+__global__ void __launch_bounds__(256, FORM == 1 ? 8 : FORM == 2 ? 5 : 4) k_lz_subtract(const T* basis, T* w, int64_t n, int64_t bs, LzState<T> s) {
+  if (*s.done) return;
+  const int i = *s.step;
+  const int64_t N = n * bs, step = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = FORM ? 1 : 4;
+  const bool narrow = N < ((int64_t)1 << 32);  // 32-bit remainders
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < (FORM ? N / 4 : N); u += U * step) {
+    if constexpr (FORM != 0) {
+      const int64_t b = FORM == 2 ? 0 : 4 * u % bs;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 1; j <= i; ++j) {
+        const float4 v = reinterpret_cast<const float4*>(basis + (int64_t)j * N)[u];
+        const float* h = s.hbuf + (int64_t)j * bs + b;
+        acc.x += v.x * h[0];
+        acc.y += v.y * h[FORM == 2 ? 0 : 1];
+        acc.z += v.z * h[FORM == 2 ? 0 : 2];
+        acc.w += v.w * h[FORM == 2 ? 0 : 3];
       }
+      float4 x = reinterpret_cast<const float4*>(w)[u];
+      x.x -= acc.x;
+      x.y -= acc.y;
+      x.z -= acc.z;
+      x.w -= acc.w;
+      reinterpret_cast<float4*>(w)[u] = x;
+    } else {
+      T acc[U];
+      const T *v[U], *h[U];
 #pragma unroll
-      for (int q = 0; q < JB; ++q) smem[q * TT + t] = acc[q];
-      team_sync();
-      for (int wd = rpp; wd > 1;) {  // tree over the row slots, all JB sums at once
-        const int h = (wd + 1) >> 1;
-        if (my_r < wd - h) {
+      for (int q = 0; q < U; ++q) {
+        const int64_t o = u + q * step < N ? u + q * step : u;  // past the end: the first one again, not stored
+        acc[q] = T(0);
+        v[q] = basis + o;
+        h[q] = s.hbuf + (narrow ? (int64_t)((uint32_t)o % (uint32_t)bs) : o % bs);
+      }
+#pragma unroll 2
+      for (int j = 1; j <= i; ++j)
 #pragma unroll
-          for (int q = 0; q < JB; ++q) smem[q * TT + t] += smem[q * TT + t + h * bc];
-        }
-        team_sync();
-        wd = h;
-      }
-      if (t < bc) {
-        for (int q = 0; q < nj; ++q) out[(int64_t)(j0 + q) * bs + b0 + t] = smem[q * TT + t];
-      }
-      team_sync();
+        for (int q = 0; q < U; ++q) acc[q] = fma(__ldg(v[q] + (int64_t)j * N), __ldg(h[q] + (int64_t)j * bs), acc[q]);
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (u + q * step < N) w[u + q * step] -= acc[q];
     }
   }
+}
+
+static unsigned lz_sweep_blocks(int64_t units, int per_sm = 8) {
+  return (unsigned)std::min<int64_t>(std::max<int64_t>(ceil_div(units, (int64_t)256), 1), (int64_t)num_sms() * per_sm);
 }
 
 // h[j][b] = sum over the CTAs of hpart: 32 interleaved sums, then a tree over them.  32 neighbouring (j, b)
@@ -602,6 +705,46 @@ __global__ void __launch_bounds__(1024) k_lz_reduce32(int nblk, int64_t bs, int6
     if (l == 0 && u0 + q0 < total) s.hbuf[u0 + q0] = h;
     __syncthreads();
   }
+}
+
+// The end of a Lanczos step, by the last CTA: subdiag[b][i] = |w| from the CTAs' sums of squares, i += 1 and
+// the stop test of lanczos_fact.cond_fun.  Without subdiag (Arnoldi) only the norms are left in nrm.
+template <class T>
+__device__ __forceinline__ void lz_step_end(const LzState<T>& s, int64_t bs, int i, T* subdiag, int max_iters, double tol,
+                                            T* scratch) {
+  __shared__ int s_any;
+  __shared__ T tot[kLzStage], red[32];
+  lz_stage(s.npart, gridDim.x, bs, tot, red, scratch);
+  if (threadIdx.x == 0) s_any = 0;
+  __syncthreads();
+  for (int64_t b = threadIdx.x; b < bs; b += blockDim.x) {
+    const T nv = sqrt(lz_total(s.npart, gridDim.x, bs, b, tot));
+    s.nrm[b] = nv;  // what V[i + 1] is divided by
+    if (subdiag) {
+      subdiag[b * (max_iters + 1) + i] = nv;
+      const T first = subdiag[b * (max_iters + 1) + 1];
+      if (nv > (T)tol * first) atomicOr(&s_any, 1);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (subdiag) {
+      const int ni = i + 1;
+      *s.step = ni;
+      *s.done = !(ni <= max_iters && (s_any || ni <= 1));
+    }
+    s.counters[2] = 0;
+  }
+}
+
+// |w| per column and the end of the step, w complete.
+template <class T>
+__global__ void __launch_bounds__(256) k_lz_finish(const T* w, int64_t n, int64_t bs, T* subdiag, int max_iters,
+                                                   double tol, LzState<T> s) {
+  if (*s.done) return;
+  __shared__ T smem[256];
+  lz_colsum<T>(n, bs, w, w, s.npart + (int64_t)blockIdx.x * bs, smem);
+  if (lz_last_block(s.counters + 2)) lz_step_end<T>(s, bs, *s.step, subdiag, max_iters, tol, smem);
 }
 
 // The last subtraction with the sums of squares of lz_colsum on the way (the same rows per thread), then
@@ -688,41 +831,26 @@ __global__ void __launch_bounds__(256, FORM == 1 ? 4 : 2) k_lz_fin(const __grid_
                        },
                        out, smem);
   }
-  if (lz_last_block(s.counters + 2)) {
-    __shared__ int s_any;
-    __shared__ float tot[kLzStage], red[32];
-    lz_stage(s.npart, gridDim.x, bs, tot, red, smem);
-    if (t == 0) s_any = 0;
-    __syncthreads();
-    for (int64_t b = t; b < bs; b += blockDim.x) {
-      const float nv = sqrt(lz_total(s.npart, gridDim.x, bs, b, tot));
-      s.nrm[b] = nv;  // what V[i + 1] is divided by
-      subdiag[b * (a.max_iters + 1) + i] = nv;
-      const float first = subdiag[b * (a.max_iters + 1) + 1];
-      if (nv > (float)tol * first) atomicOr(&s_any, 1);
-    }
-    __syncthreads();
-    if (t == 0) {
-      const int ni = i + 1;
-      *s.step = ni;
-      *s.done = !(ni <= a.max_iters && (s_any || ni <= 1));
-      s.counters[2] = 0;
-    }
-  }
+  if (lz_last_block(s.counters + 2)) lz_step_end<float>(s, bs, i, subdiag, a.max_iters, tol, smem);
 }
 
 // Which projection form a run of the FP32 method uses, and its launch shape (nb: the partials' capacity).
 struct LzForm {
-  int form = 2;  // 0: k_lz_proj1, 1: k_lz_projq, 2: k_lz_projx
+  int form = 2;  // 0: k_lz_proj1, 1: k_lz_projq, 2: k_lz_projx, 3: passes of their own
   int blocks = 1;
   int64_t chunk = 0;
   size_t smem = 0;
 };
+// Blocks of more entries than this that have no staged form take their passes one by one.  ms for 24 steps of an
+// FP32 block, staged in teams / pass by pass: 50,000 x 3 1.60 / 1.87, 100,000 x 3 2.08 / 2.11, 50,000 x 7 2.70 / 2.55,
+// 100,000 x 10 4.28 / 3.59, 1,000,000 x 7 24.7 / 13.2.
+constexpr int64_t kLzSplit = 320 * 1024;
 constexpr size_t kLzRunSmem = 160 * 1024, kLzProj1Smem = 220 * 1024;
 static int lz_form(const float* basis, int64_t n, int64_t bs, int nb, int64_t slots, LzForm& f) {
   const bool al = (uintptr_t)basis % 16 == 0;
   f.blocks = nb;
   f.chunk = ceil_div(n, (int64_t)nb);
+  if (n * bs > kLzSplit) f.form = 3;
   int64_t step = 0;
   if (bs == 1 && n % 4 == 0 && al) step = 128;
   else if (bs >= 4 && bs <= 128 && (bs & (bs - 1)) == 0 && al) step = 128 / bs;
@@ -761,14 +889,34 @@ static void lz_project(const LzForm& f, const LzStep& a, int i, cudaStream_t st)
 static int lz_step_f32(const LzForm& f, const LzStep& a, int i, int nb, float* diag, float* subdiag, double tol,
                        cudaStream_t st) {
   const unsigned rb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * a.bs, 32), 4096));
-  k_lz_alpha<<<nb, 256, 0, st>>>(a.w, a.vi, a.n, a.bs, diag, a.max_iters, a.s);
-  lz_project<LZ_TERMS_PROJ>(f, a, i, st);
-  k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
-  lz_project<LZ_SUB_PROJ>(f, a, i, st);
-  k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
   // the 128-bit form where lz_colsum takes it: blocks of 4, 8, ... columns and single ones with n % 4 == 0
   const bool quads = (uintptr_t)a.basis % 16 == 0 && (uintptr_t)a.w % 16 == 0 &&
                      ((a.bs == 1 && a.n % 4 == 0) || (a.bs % 4 == 0 && a.bs <= 1024));
+  auto subtract = [&]() {
+    const int64_t N = a.n * a.bs;
+    if (!quads) k_lz_subtract<float, 0><<<lz_sweep_blocks(N, 4), 256, 0, st>>>(a.basis, a.w, a.n, a.bs, a.s);
+    else if (a.bs == 1) k_lz_subtract<float, 2><<<lz_sweep_blocks(N / 4), 256, 0, st>>>(a.basis, a.w, a.n, a.bs, a.s);
+    else k_lz_subtract<float, 1><<<lz_sweep_blocks(N / 4), 256, 0, st>>>(a.basis, a.w, a.n, a.bs, a.s);
+  };
+  k_lz_alpha<<<nb, 256, 0, st>>>(a.w, a.vi, a.n, a.bs, diag, a.max_iters, a.s);
+  if (f.form == 3) {
+    k_lz_terms<<<lz_sweep_blocks(a.n * a.bs), 256, 0, st>>>(a);
+    k_lz_project<float><<<nb, kLzTeam, 0, st>>>(a.basis, a.w, a.n, a.bs, a.slots, a.s);
+    k_lz_reduce32<<<rb, 1024, 0, st>>>(nb, a.bs, a.slots, a.s);
+    subtract();
+    k_lz_project<float><<<nb, kLzTeam, 0, st>>>(a.basis, a.w, a.n, a.bs, a.slots, a.s);
+    k_lz_reduce32<<<rb, 1024, 0, st>>>(nb, a.bs, a.slots, a.s);
+    if (!quads) {
+      subtract();
+      k_lz_finish<float><<<nb, 256, 0, st>>>(a.w, a.n, a.bs, subdiag, a.max_iters, tol, a.s);
+      return COLAGB_OK;
+    }
+  } else {
+    lz_project<LZ_TERMS_PROJ>(f, a, i, st);
+    k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
+    lz_project<LZ_SUB_PROJ>(f, a, i, st);
+    k_lz_reduce32<<<rb, 1024, 0, st>>>(f.blocks, a.bs, a.slots, a.s);
+  }
   if (!quads) k_lz_fin<0><<<nb, 256, 0, st>>>(a, subdiag, tol);
   else if (a.bs == 1) k_lz_fin<2><<<nb, 256, 0, st>>>(a, subdiag, tol);
   else k_lz_fin<1><<<nb, 256, 0, st>>>(a, subdiag, tol);
@@ -792,7 +940,9 @@ static int lz_step_f32(const LzForm& f, const LzStep& a, int i, int nb, float* d
 // unit is a float4 for FP32 with bs = 1 or a multiple of 4 on 16-byte boundaries, else one entry.
 //
 // It replaced norm, dot, three-term update and four sweeps, 12 launches a step beside the operator, with one
-// dependent load per slot and thread.
+// dependent load per slot and thread.  Long vectors take the same two passes through k_lz_project and
+// k_lz_subtract (gs_plan says from where on): a run's second read misses the caches then, and 512 threads with a
+// run of w in shared memory keep fewer loads in flight than plain sweeps.
 enum { GS_PROJECT = 0, GS_SUB_PROJ = 1, GS_SUB_NORM = 2 };
 constexpr int kGsThreads = 512;
 
@@ -993,32 +1143,8 @@ __global__ void __launch_bounds__(kGsThreads) k_lz_gs(const __grid_constant__ Gs
       }
     }
   }
-  if (MODE == GS_SUB_NORM && lz_last_block(s.counters + 2)) {
-    // subdiag[b][i] = |w| ; i += 1 ; stop test of lanczos_fact.cond_fun
-    __shared__ int s_any;
-    __shared__ T tot[kLzStage], bred[32];
-    lz_stage(s.npart, gridDim.x, g.bs, tot, bred, red);
-    if (t == 0) s_any = 0;
-    __syncthreads();
-    for (int64_t b = t; b < g.bs; b += kGsThreads) {
-      const T nv = sqrt(lz_total(s.npart, gridDim.x, g.bs, b, tot));
-      s.nrm[b] = nv;
-      if (g.subdiag) {
-        g.subdiag[b * (g.max_iters + 1) + i] = nv;
-        const T first = g.subdiag[b * (g.max_iters + 1) + 1];
-        if (nv > (T)g.tol * first) atomicOr(&s_any, 1);
-      }
-    }
-    __syncthreads();
-    if (t == 0) {
-      if (g.subdiag) {
-        const int ni = i + 1;
-        *s.step = ni;
-        *s.done = !(ni <= g.max_iters && (s_any || ni <= 1));
-      }
-      s.counters[2] = 0;
-    }
-  }
+  if (MODE == GS_SUB_NORM)
+    if (lz_last_block(s.counters + 2)) lz_step_end<T>(s, g.bs, i, g.subdiag, g.max_iters, g.tol, red);
 }
 
 // h[j][b] = sum over the CTAs of hpart, 32 neighbouring sums per block and eight threads each.  What
@@ -1061,7 +1187,7 @@ constexpr size_t kGsSmem = 200 * 1024;
 // Launch plan of k_lz_gs for one run of the method.
 struct GsPlan {
   int vec = 1, run = 0, blocks = 1;
-  bool staged = true;
+  bool staged = true, split = false;  // split: passes of their own on `blocks` CTAs
   size_t smem = 0;
 };
 
@@ -1082,6 +1208,14 @@ static GsPlan gs_plan(const T* basis, int64_t n, int64_t bs, int max_blocks) {
     p.staged = false;
     p.vec = 1;
     p.smem = (size_t)kGsThreads * sizeof(T);
+  }
+  // Long vectors: pass by pass, unless the columns leave a quarter of a team idle there.  ms for 24 steps, FP64
+  // Lanczos, k_lz_gs / pass by pass: 100,000 x 10 5.85 / 6.3, 400,000 x 3 6.7 / 6.2, 50,000 x 33 11.6 / 9.2, 100,000 x 20
+  // 18.9 / 10.2, 1,000,000 x 33 194 / 108; FP32 Arnoldi, 100,000 x 10 2.8 / 3.0, 50,000 x 33 6.6 / 4.7, 400,000 x 10
+  // 19.4 / 7.6.
+  if (N > 1100000 && (bs >= kLzTeam || kLzTeam / bs * bs >= kLzTeam * 3 / 4)) {
+    p.split = true;
+    p.blocks = max_blocks;
   }
   return p;
 }
@@ -1108,6 +1242,16 @@ static int gs_step(const GsPlan& p, const T* basis, T* w, int64_t n, int64_t bs,
                    int max_iters, double tol, const LzState<T>& s, cudaStream_t st) {
   GsArgs<T> a{basis, w, n * bs, bs, p.run, (int64_t)max_iters + 2, subdiag, max_iters, tol, s};
   const unsigned rb = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div((int64_t)(i + 1) * bs, 32), 4096));
+  if (p.split) {
+    const unsigned sweep = lz_sweep_blocks(n * bs, 4);
+    for (int pass = 0; pass < 2; ++pass) {
+      k_lz_project<T><<<p.blocks, kLzTeam, 0, st>>>(basis, w, n, bs, a.slots, s);
+      k_lz_reduce_h<T><<<rb, 256, 0, st>>>(p.blocks, bs, a.slots, pass ? (T*)nullptr : diag, H, !pass, max_iters, s);
+      k_lz_subtract<T, 0><<<sweep, 256, 0, st>>>(basis, w, n, bs, s);
+    }
+    k_lz_finish<T><<<p.blocks, 256, 0, st>>>(w, n, bs, subdiag, max_iters, tol, s);
+    return COLAGB_OK;
+  }
   COLAGB_TRY((launch_gs<T, GS_PROJECT>(p, a, st)));
   k_lz_reduce_h<T><<<rb, 256, 0, st>>>(p.blocks, bs, a.slots, diag, H, 1, max_iters, s);
   COLAGB_TRY((launch_gs<T, GS_SUB_PROJ>(p, a, st)));
