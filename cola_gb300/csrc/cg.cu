@@ -457,13 +457,26 @@ __global__ void k_pupdate(T* P, const T* R, const T* Z, const T* dinv, int64_t n
 // One step after Ap in a single launch (P = identity or Diagonal), by one cluster of kTailCtas CTAs (Ap stands for
 // AP + shift p: the scalar part of A = B + c I is added here instead of by a launch of its own):
 //   <p, Ap>, alpha ; x += alpha p, r -= alpha Ap, |r|^2, <r, z>, beta, stop test ; p = z + beta p,
-// the CTAs' column sums added through distributed shared memory in rank order by every CTA.  For blocks of up
-// to kTailMax entries the step is bound by the launches and the last-block reductions of k_alpha, k_update
-// and k_pupdate (8.3 + 11.5 + 3.4 us at 7680 x 8, here 9.7 us); larger ones want all SMs.
+// the CTAs' column sums added through distributed shared memory in rank order by every CTA.  Smaller blocks are
+// bound by the launches and the last-block reductions of k_alpha, k_update and k_pupdate (8.3 + 11.5 + 3.4 us at
+// 7680 x 8, here 9.7 us); larger ones want all SMs (tail_max).
 constexpr int kTailCtas = 16, kTailThreads = 1024;
-// (FP64: 16 SMs have 32 multiply-adds a cycle between them, six per entry.)
-template <class T> constexpr int64_t kTailMax = std::is_same<T, double>::value ? 48 * 1024 : 512 * 1024;
 constexpr int64_t kTailMaxCols = 512;
+
+// The most entries of a block that goes through k_cg_tail: us a step of a Diagonal operator, one launch / three, without
+// a preconditioner.  FP32, shuffle sums: 1 column 196,608 entries 20.6 / 20.1, 131,072 17.6 / 20.0; 8 columns 327,680
+// 26.6 / 26.2; 16 columns 460,000 32.1 / 34.5; 32 columns 524,288 36 / 51.  Other column counts: 3 columns 131,072
+// 22.4 / 22.4; 12 columns 262,144 32.3 / 31.3; 50 columns 524,288 42 / 87.  FP64, whose 16 SMs have 32 multiply-adds a
+// cycle between them: 1 column 24,000 22.9 / 22.4, 2 columns 32,000 22.7 / 23.2, 40,000 24.3 / 23.2, 8 columns 48,000
+// 23.5 / 23.9.  A scalar part that the tail adds saves a launch of 3 to 4 us
+// besides (256 x 256 x 4 Kronecker + c I, 262,144 entries: 51.4 / 54.6).
+template <class T>
+static int64_t tail_max(int64_t k, bool scalar_part) {
+  if (std::is_same<T, double>::value) return (scalar_part || k > 2 ? 48 : k == 2 ? 32 : 24) * 1024;
+  const bool shuffles = k <= 32 && (k & (k - 1)) == 0;
+  const int64_t most = shuffles ? (k >= 16 ? 512 : k >= 8 ? 320 : 180) : k >= 32 ? 512 : k >= 16 ? 320 : k >= 8 ? 256 : 128;
+  return std::min<int64_t>(most + (scalar_part ? 96 : 0), 512) * 1024;
+}
 
 // Column sums of the CTA, as block_col_sums, for the tail: with a power-of-two number of FP32 columns up to 32
 // the lanes of a column are added by shuffles and the warps in one more step (the general tree passes ten
@@ -629,8 +642,8 @@ static int launch_tail(T* X, int64_t ldx, T* R, T* P, const T* AP, T shift, cons
 
 // Whether the step's tail runs as one cluster here (sizes, and the device can schedule the cluster).
 template <class T, int PK>
-static bool tail_ok(int64_t n, int64_t k) {
-  if (n * k > kTailMax<T> || k > kTailMaxCols) return false;
+static bool tail_ok(int64_t n, int64_t k, bool scalar_part) {
+  if (n * k > tail_max<T>(k, scalar_part) || k > kTailMaxCols) return false;
   auto* f = k_cg_tail<T, PK>;
   const size_t smem = sizeof(T) * ((PK == 1 ? 2 : 1) * kTailThreads + 5 * k);
   static_assert(sizeof(T) * (2 * kTailThreads + 5 * kTailMaxCols) <= 48 * 1024, "above the default limit");
@@ -1182,11 +1195,10 @@ static int run_generic(const colagb_op* A, const colagb_op* P, const CgPlan& pl,
   COLAGB_CUDA(cudaGetLastError());
   int h_done[2] = {0, 0};
   const int every = prm.check_every > 0 ? prm.check_every : 16;
-  const bool tail = pl.pk == 0 ? tail_ok<T, 0>(n, k) : pl.pk == 1 && tail_ok<T, 1>(n, k);
   // the node whose product a step forms, and what the tail adds to it
   int a_node = A->root;
   T shift = T(0);
-  if (tail && A->nodes[a_node].kind == COLAGB_OP_SUM && A->children[a_node].size() == 2)
+  if (A->nodes[a_node].kind == COLAGB_OP_SUM && A->children[a_node].size() == 2)
     for (int e = 0; e < 2; ++e) {
       const int other = A->children[A->root][1 - e];
       const colagb_op_node& c = A->nodes[A->children[A->root][e]];
@@ -1195,6 +1207,9 @@ static int run_generic(const colagb_op* A, const colagb_op* P, const CgPlan& pl,
         a_node = other;
       }
     }
+  const bool folds = a_node != A->root;
+  const bool tail = pl.pk == 0 ? tail_ok<T, 0>(n, k, folds) : pl.pk == 1 && tail_ok<T, 1>(n, k, folds);
+  if (!tail) a_node = A->root;
   // One step of the loop: Ap, alpha, x / r update (+ z = P r and gamma for a general P), p update.
   // Every kernel reads the device stop flag and does nothing once it is set, so a block of steps may
   // run past convergence or max_iters (the device counts the steps and enforces max_iters).
