@@ -218,7 +218,7 @@ def solve_batched(A: BatchedCSR, B: torch.Tensor, precond: str = "jacobi", tol: 
             schedules); X and the per-system tensors of info are then ready in stream order and
             info["sweeps"] is None.  The scratch buffer is per stream, so solves on other streams may
             run meanwhile.
-        spin_limit: naps a CTA of the "grid" schedule may take in one grid barrier before the solve
+        spin_limit: polls a CTA of the "grid" schedule may take in one grid barrier before the solve
             gives up with COLAGB_ERR_TIMEOUT (a ColagbError); 0 keeps the library default (seconds).
         matvec: "fp32" -- the inner CG multiplies by the FP32 values; "bf16" -- by BF16 off-diagonal
             values with an FP32 diagonal made consistent with them (within 2^-9 of A in the energy norm
