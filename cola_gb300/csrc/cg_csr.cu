@@ -13,7 +13,7 @@
 // previous p (double buffered, each CTA publishes its own) from L2 and combines them on the fly.
 //
 // It is bound by the two barriers (1.3 us each on 152 CTAs), the L2 round trips after them and, in FP64, by
-// the arithmetic itself (64 to 80 cycles of a scheduler per warp instruction: all 512 threads take rows, so
+// the arithmetic itself (64 cycles of a scheduler per warp instruction: all 512 threads take rows, so
 // that their loads overlap, but 128 of them form the sums and the divisions).  Before, 16 CTAs of one cluster ran matrices up to
 // 32 MB: 37 us a step for 256 x 256 5-point FP64 with Jacobi; now 11.6 (FP32 6.1; the barriers and round
 // trips alone take 5.6).

@@ -134,7 +134,7 @@ __device__ __forceinline__ void d_tail(const float4 (&a)[N], const float* P, int
 
 // <A row, p> over one warp; the result is in every lane.  Ar: the row (ns floats); P0: copy 0 of p,
 // cs: the copy length.  Each lane keeps eight independent 128-bit loads of A in flight (4 KB per
-// warp, four 256-thread blocks per SM): the matvec streams HBM and is bound by how many bytes are in
+// warp, 32 warps per SM): the matvec streams HBM and is bound by how many bytes are in
 // flight, not by instructions (with 256-thread CTAs: four quads per lane and 3 blocks reached 0.46 of the copy bandwidth,
 // four quads and 4 blocks 0.64, eight quads and 4 blocks 0.78; an L2 prefetch ahead of the loads
 // lowered each).

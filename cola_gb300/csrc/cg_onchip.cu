@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kOT, 1) k_onchip_pcg(const __grid_constant__ O
 // (7 clusters = 112 of the 152 SMs at 224 KB of shared memory per CTA); on each remaining SM one
 // 512-thread CTA solves whole systems alone, with the same algorithm and stop rule, its vectors in
 // global memory.  It claims systems from the on-chip kernel's counter while more than `reserve`
-// remain unclaimed, so that the clusters (about ten times faster per system) finish the tail.
+// remain unclaimed, so that the clusters (kSpareRatio, 28 times, faster per system) finish the tail.
 //
 // Layout per CTA: the system's rows padded to np (a multiple of 4 * kST * kRowBatch) in the strip
 // layout of the on-chip schedule with the CTA as the whole "cluster" (S = np / 4 float4 groups), so
