@@ -877,7 +877,7 @@ extern "C" int colagb_cg_batched_csr_solve(const colagb_batched_csr* A, const do
     a.gb.err = reinterpret_cast<int*>(w.bar + 2);
     a.gb.spin_limit = params->spin_limit > 0 ? params->spin_limit : kDefaultSpinLimit;
     const size_t smem = batched_smem(S);
-    COLAGB_CUDA(set_smem_limit(k_batched_ir, batched_smem(kMaxBatch)));
+    if (smem > 48 * 1024) COLAGB_CUDA(set_smem_limit(k_batched_ir, batched_smem(kMaxBatch)));
     int occ = 0;
     COLAGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batched_ir, kThreads, smem));
     if (occ < 1) return fail(COLAGB_ERR_UNSUPPORTED, "batched CG kernel cannot be resident");

@@ -571,7 +571,7 @@ extern "C" int colagb_cg_dense_batched_solve(int64_t num_systems, const int32_t*
   a.gb.spin_limit = kDefaultSpinLimit;
   cudaStream_t st = as_stream(stream);
   const size_t smem = dense_batch_smem(a.S);
-  COLAGB_CUDA(set_smem_limit(k_dense_batched_cg, dense_batch_smem(kDBMaxSystems)));
+  if (smem > 48 * 1024) COLAGB_CUDA(set_smem_limit(k_dense_batched_cg, dense_batch_smem(kDBMaxSystems)));
   int occ = 0;
   COLAGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_dense_batched_cg, kDBThreads, smem));
   if (occ < 1) return fail(COLAGB_ERR_UNSUPPORTED, "dense batched CG kernel cannot be resident");

@@ -47,7 +47,8 @@ __device__ __forceinline__ bool lz_last_block(unsigned int* counter) {
 
 // Per-probe column reduction over rows of an n x bs block: f(r, b) summed per b.
 // Block layout: threads = (rows_per_pass x bsc), bsc = min(bs, 256).
-template <class T, class F>
+// U: rows in flight.
+template <class T, int U = 1, class F>
 __device__ __forceinline__ void lz_partials(int64_t n, int64_t bs, F f, T* out, T* smem) {
   const int t = threadIdx.x;
   for (int64_t b0 = 0; b0 < bs; b0 += blockDim.x) {
@@ -56,7 +57,7 @@ __device__ __forceinline__ void lz_partials(int64_t n, int64_t bs, F f, T* out, 
     const int my_b = t % bc, my_r = t / bc;
     T acc = T(0);
     if (my_r < rpp)
-#pragma unroll 4
+#pragma unroll U
       for (int64_t r = (int64_t)blockIdx.x * rpp + my_r; r < n; r += (int64_t)rpp * gridDim.x) acc += f(r, b0 + my_b);
     smem[t] = acc;
     __syncthreads();
@@ -166,7 +167,7 @@ __device__ __forceinline__ void lz_colsum(int64_t n, int64_t bs, const T* a, con
       return;
     }
   }
-  lz_partials<T>(n, bs, [&](int64_t r, int64_t b) { return a[r * bs + b] * c[r * bs + b]; }, out, smem);
+  lz_partials<T, 4>(n, bs, [&](int64_t r, int64_t b) { return a[r * bs + b] * c[r * bs + b]; }, out, smem);
 }
 
 // Sum over the nb per-CTA partials of column b, formed by the whole block (all threads get it).
@@ -1223,7 +1224,7 @@ static GsPlan gs_plan(const T* basis, int64_t n, int64_t bs, int max_blocks) {
 template <class T, int VEC, int MODE, bool STAGED>
 static int launch_gs_form(const GsPlan& p, const GsArgs<T>& a, cudaStream_t st) {
   auto* f = k_lz_gs<T, VEC, MODE, STAGED>;
-  COLAGB_CUDA(set_smem_limit(f, kGsSmem));
+  if (p.smem > 48 * 1024) COLAGB_CUDA(set_smem_limit(f, kGsSmem));
   f<<<p.blocks, kGsThreads, p.smem, st>>>(a);
   return COLAGB_OK;
 }
@@ -1853,7 +1854,7 @@ static int tridiag_eig(const R* a, const R* b, int64_t m, int64_t batch, R* eval
   const int two = smem2 <= kTriSmem;
   const size_t smem = two ? smem2 : smem1;
   if (smem > kTriSmem) return fail(COLAGB_ERR_INVALID, "tridiagonal eigensolver: m too large");
-  COLAGB_CUDA(set_smem_limit(k_tridiag_ql<R>, kTriSmem));
+  if (smem > 48 * 1024) COLAGB_CUDA(set_smem_limit(k_tridiag_ql<R>, kTriSmem));
   const size_t smem_rot = (size_t)m * kRotRows * sizeof(R);
   if (evecs && smem_rot <= kTriSmem) {
     // eigenvectors: QL records its rotations (one thread generates them serially), then many CTAs
@@ -1871,7 +1872,7 @@ static int tridiag_eig(const R* a, const R* b, int64_t m, int64_t batch, R* eval
     k_tridiag_ql<R><<<(unsigned)batch, 128, smem, st>>>(a, b, m, two, evals, first_row, nullptr, status, rec, rec_i,
                                                         rec_n, rec_perm, cap);
     COLAGB_CUDA(cudaGetLastError());
-    COLAGB_CUDA(set_smem_limit(k_tridiag_apply<R>, kTriSmem));
+    if (smem_rot > 48 * 1024) COLAGB_CUDA(set_smem_limit(k_tridiag_apply<R>, kTriSmem));
     k_tridiag_apply<R><<<dim3((unsigned)ceil_div(m, (int64_t)kRotRows), (unsigned)batch), kRotRows, smem_rot, st>>>(
         rec, rec_i, rec_n, rec_perm, m, cap, evecs);
     COLAGB_CUDA(cudaGetLastError());
