@@ -132,7 +132,7 @@ __device__ __forceinline__ void dc_rows(const S* A, int64_t lda, int R, int n, i
   for (int rb = wr * RB; rb < R; rb += WR * RB) {
     // One FP32 column: a quad's four products are added to each other before they join the lane's sum, so that
     // a lane's chain has a link per quad.  (A link per product, 32 of them at n = 2048, left the solutions at
-    // condition 100 1.15 times further from the exact ones.)
+    // condition 1000 1.15 times further from the exact ones.)
     constexpr bool QUADS = std::is_same<T, float>::value && K == 1;
     T acc[V];
 #pragma unroll
