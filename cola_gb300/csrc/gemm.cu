@@ -479,12 +479,12 @@ static int launch_form(GemmArgs<T, S>& g, cudaStream_t st) {
 template <class T, class S>
 static bool gemm_async(const GemmArgs<T, S>& g) { return g.avec && g.xvec && g.K % 4 == 0 && g.N % 4 == 0; }
 
-template <class T, class S, int BM, int BN, int BK, int WM, int WN, int WK, int ST>
+template <class T, class S, int BM, int BN, int BK, int WM, int WN, int WK, int ST, bool MAY_ASYNC = true>
 static int launch_tile(GemmArgs<T, S>& g, int split, bool xk, cudaStream_t st) {
   g.mtiles = ceil_div(g.M, (int64_t)BM);
   g.split = split;
   if (xk) return launch_form<T, S, BM, BN, BK, WM, WN, WK, 2, true, false>(g, st);
-  if constexpr (gemm_async_types<T, S>)
+  if constexpr (gemm_async_types<T, S> && MAY_ASYNC)
     if (gemm_async(g)) return launch_form<T, S, BM, BN, BK, WM, WN, WK, ST, false, true>(g, st);
   return launch_form<T, S, BM, BN, BK, WM, WN, WK, 2, false, false>(g, st);
 }
@@ -549,7 +549,7 @@ int dense_contract(const S* A, int64_t lda, int64_t M, int64_t K, const T* X, in
     }
     if (g.N > 32 && (t64 >= sms || (g.N <= 64 && K >= 512))) {
       if constexpr (!std::is_same<T, S>::value)
-        if (!gemm_async(g)) return launch_tile<T, S, 64, 64, 16, 2, 2, 2, 3>(g, split_for(64, 64, 16), xk, st);
+        if (!gemm_async(g)) return launch_tile<T, S, 64, 64, 16, 2, 2, 2, 2, false>(g, split_for(64, 64, 16), xk, st);
       return launch_tile<T, S, 64, 64, 32, 2, 1, 2, 3>(g, split_for(64, 64, 32), xk, st);
     }
     if (g.N > 16 && K >= 512) return launch_tile<T, S, 64, 32, 64, 2, 1, 4, 3>(g, split_for(64, 32, 64), xk, st);
