@@ -5,7 +5,6 @@ stop at |r| <= tol |r0| + tol with |r0| the residual of the scaled system, and a
 most |r| / lambda_min.  The matrices are diagonally dominant by `margin`, so lambda_min >= margin."""
 import pytest
 import torch
-from torch.profiler import ProfilerActivity, profile
 
 import cola_gb300 as cola
 from cola_gb300.linalg import cg
@@ -32,13 +31,6 @@ def _matrix(n, pairs, spread, dtype, full_row=0):
 F32, F64 = torch.float32, torch.float64
 
 
-@pytest.fixture(scope="module", autouse=True)
-def _first_profile():  # the profiler's first use records nothing
-    with profile(activities=[ProfilerActivity.CUDA]):
-        torch.zeros(1, device="cuda")
-        torch.cuda.synchronize()
-
-
 @pytest.mark.parametrize("dtype,n,pairs,spread,full_row,kernel", [
     (F32, 8192, 2, 90, 0, "k_cg_fused"), (F32, 8193, 2, 90, 0, "k_cg_csr"), (F32, 2000, 12, 90, 0, "k_cg_csr"),
     (F64, 8192, 2, 90, 0, "k_cg_csr"),
@@ -50,19 +42,14 @@ def _first_profile():  # the profiler's first use records nothing
     (F64, 5000, 2, 50, 240, "k_cg_csr"), (F64, 5000, 2, 50, 300, "k_cg_fused"), (F64, 70000, 2, 50, 70000, "k_cg_fused"),
     (F32, 40000, 2, 50, 30000, "k_cg_csr"), (F32, 40000, 2, 50, 40000, "k_cg_fused")])
 @pytest.mark.parametrize("start", [False, True])
-def test_route_and_solution(dtype, n, pairs, spread, full_row, kernel, start):
+def test_route_and_solution(kernels_of, dtype, n, pairs, spread, full_row, kernel, start):
     A, d = _matrix(n, pairs, spread, dtype, full_row)
     g = torch.Generator("cuda").manual_seed(n)
     b = torch.randn(n, generator=g, device="cuda", dtype=torch.float64).to(dtype)
     x0 = torch.randn(n, generator=g, device="cuda", dtype=torch.float64).to(dtype) if start else None
     P = None if start else cola.Diagonal((1.0 / d).to(dtype))
     tol = 1e-4 if dtype == F32 else 1e-10
-    cg(cola.PSD(A), b, P=P, tol=tol, max_iters=400)
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        x, info = cg(cola.PSD(A), b, x0=x0, P=P, tol=tol, max_iters=400)
-        torch.cuda.synchronize()
-    names = [e.key for e in prof.key_averages()]
+    (x, info), names = kernels_of(lambda: cg(cola.PSD(A), b, x0=x0, P=P, tol=tol, max_iters=400))
     ran = [k for k in ("k_cg_csr", "k_cg_fused") if any(k in name for name in names)]
     assert ran[-1:] == [kernel] and info["fused"], ran
     assert info["iterations"] - 1 < 400

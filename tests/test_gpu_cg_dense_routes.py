@@ -2,7 +2,6 @@
 of the rule; both give the solution (cond 1.5: the true residual stays within a few roundings of 2 tol)."""
 import pytest
 import torch
-from torch.profiler import ProfilerActivity, profile
 
 import cola_gb300 as cola
 from cola_gb300.linalg import cg
@@ -10,16 +9,9 @@ from cola_gb300.linalg import cg
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module", autouse=True)
-def _first_profile():  # the profiler's first use records nothing
-    with profile(activities=[ProfilerActivity.CUDA]):
-        torch.zeros(1, device="cuda")
-        torch.cuda.synchronize()
-
-
 @pytest.mark.parametrize("n,jacobi,kernel", [(16000, False, "k_cg_dense"), (16200, False, "k_cg_fused"),
                                              (16200, True, "k_cg_dense"), (16201, False, "k_cg_dense")])
-def test_long_vectors(n, jacobi, kernel):
+def test_long_vectors(kernels_of, n, jacobi, kernel):
     # a rank-one update of the identity: eigenvalues 1 and 1 + 0.5
     v = torch.randn(n, generator=torch.Generator("cuda").manual_seed(n), device="cuda")
     v /= v.norm()
@@ -27,10 +19,7 @@ def test_long_vectors(n, jacobi, kernel):
     A.diagonal().add_(1.0)
     b = torch.randn(n, generator=torch.Generator("cuda").manual_seed(1), device="cuda")
     P = cola.Diagonal(1.0 / A.diagonal()) if jacobi else None
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        x, info = cg(cola.PSD(cola.Dense(A)), b, P=P, tol=1e-5, max_iters=50)
-        torch.cuda.synchronize()
-    names = [e.key for e in prof.key_averages()]
+    (x, info), names = kernels_of(lambda: cg(cola.PSD(cola.Dense(A)), b, P=P, tol=1e-5, max_iters=50))
     assert any(kernel in name for name in names), names
     assert info["fused"] and info["iterations"] < 20
     xd, bd, vd = x.double(), b.double(), v.double()

@@ -4,7 +4,6 @@ the solution is known: cond 2 contracts the error by 0.18 a step, and the residu
 with |r0| = 1, bounds the error by 2 tol |b| / 1 plus the 30 steps' roundings."""
 import pytest
 import torch
-from torch.profiler import ProfilerActivity, profile
 
 import cola_gb300 as cola
 from cola_gb300.linalg import cg
@@ -13,20 +12,13 @@ pytestmark = pytest.mark.gpu
 F32, F64 = torch.float32, torch.float64
 
 
-@pytest.fixture(scope="module", autouse=True)
-def _first_profile():  # the profiler's first use records nothing
-    with profile(activities=[ProfilerActivity.CUDA]):
-        torch.zeros(1, device="cuda")
-        torch.cuda.synchronize()
-
-
 # entries (of 1024) up to which a block takes one launch
 @pytest.mark.parametrize("dtype,k,scalar,limit", [
     (F32, 1, False, 180), (F32, 1, True, 276), (F32, 8, False, 320), (F32, 16, False, 512), (F32, 16, True, 512),
     (F32, 3, False, 128), (F32, 3, True, 224), (F32, 12, False, 256), (F32, 20, False, 320), (F32, 33, False, 512),
     (F64, 1, False, 24), (F64, 2, False, 32), (F64, 3, False, 48), (F64, 1, True, 48)])
 @pytest.mark.parametrize("jacobi", [False, True])
-def test_limits(dtype, k, scalar, limit, jacobi):
+def test_limits(kernels_of, dtype, k, scalar, limit, jacobi):
     u = 2.0 ** -24 if dtype == F32 else 2.0 ** -53
     tol = 1e-5 if dtype == F32 else 1e-11
     for n, one in ((limit * 1024 // k, True), (limit * 1024 // k + 1, False)):
@@ -36,10 +28,8 @@ def test_limits(dtype, k, scalar, limit, jacobi):
             op = op + 0.5 * cola.I_like(op)
         b = torch.randn(n, k, generator=torch.Generator("cuda").manual_seed(k), device="cuda", dtype=F64).to(dtype)
         P = cola.Diagonal(torch.linspace(1.0, 0.9, n, device="cuda", dtype=F64).to(dtype)) if jacobi else None
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            x, info = cg(cola.PSD(op), b, P=P, tol=tol, max_iters=100)
-            torch.cuda.synchronize()
-        assert any("k_cg_tail" in e.key for e in prof.key_averages()) == one
+        (x, info), names = kernels_of(lambda: cg(cola.PSD(op), b, P=P, tol=tol, max_iters=100))
+        assert any("k_cg_tail" in name for name in names) == one
         assert not info["fused"] and info["iterations"] - 1 <= 30
         exact = b.double() / (d.to(dtype).double() + (0.5 if scalar else 0.0))[:, None]
         err = (x.double() - exact).norm(dim=0) / b.double().norm(dim=0)
